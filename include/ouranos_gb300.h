@@ -197,9 +197,13 @@ int ouranos_rt_last_sweep_ms(const ouranos_rt* rt, double* ms, int* kernels);
  * directions per warp, with cells_x * cells_y * dirs == 32 (one lane per cell),
  * or == 16 for cells of 9 or more dofs (2-D Q2+, 3-D Q2): two lanes share each
  * cell solve, or 1 x 1 x 1: one warp per cell (every order; the only tiling
- * of 2-D Q5 and 3-D Q3..Q5).  0s = the default (one direction per warp; 2-D
- * 32 x 1, 3-D 4 x 8; two lanes per cell and 16 cells where allowed: 2-D
- * 16 x 1, 3-D 4 x 4; one warp per cell for 2-D Q5 and 3-D Q3..Q5). */
+ * of 2-D Q5 and 3-D Q3..Q5).  0s = the default: the library picks the number of
+ * lanes that share a cell by DG order and problem size, and get_tiling reports the
+ * nominal tiling of the order (one direction per warp; 2-D 32 x 1, 3-D 4 x 8; two
+ * lanes per cell and 16 cells where allowed: 2-D 16 x 1, 3-D 4 x 4; one warp per
+ * cell for 2-D Q5 and 3-D Q3..Q5).  2-D Q3 and Q4 and 3-D Q2 accept the same
+ * tilings but choose their lanes themselves under all of them but 1 x 1 x 1.
+ * Every tiling gives the same bits. */
 int ouranos_rt_set_tiling(ouranos_rt* rt, int cells_x, int cells_y, int dirs_per_warp);
 int ouranos_rt_get_tiling(const ouranos_rt* rt, int* cells_x, int* cells_y, int* dirs_per_warp);
 /* Spin limit of the in-kernel dependency waits, in nanoseconds (default 2 s).

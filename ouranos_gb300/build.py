@@ -20,6 +20,10 @@ GENCODE = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = ["quadrature.cpp", "fe.cpp", "operator.cu", "solvers.cu", "vec.cu",
            "sweep_f64.cu", "sweep_f32.cu", "sweep_df64.cu", "sweep_wide_f64.cu", "sweep_wide_f32.cu",
            "sweep_wide_df64.cu", "sweep_batch_f64.cu", "sweep_batch_f32.cu",
+           "sweep_lane_f64.cu", "sweep_lane_f32.cu", "sweep_lane_df64.cu",
+           "sweep_form_batch_f64.cu", "sweep_form_batch_f32.cu",
+           "sweep_group_f64_2d.cu", "sweep_group_f64_3d.cu", "sweep_group_f32_2d.cu", "sweep_group_f32_3d.cu",
+           "sweep_group_df64_2d.cu", "sweep_group_df64_3d.cu",
            "batch.cu", "noalloc.cu", "cnn.cu", "precond.cu", "dsa.cu", "contract_tc.cu", "contract_oz.cu", "cnn_tc.cu"]
 
 

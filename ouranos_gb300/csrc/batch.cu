@@ -39,8 +39,8 @@ constexpr size_t kMaxGraphs = 64;         // captured Apply graphs kept per batc
 constexpr size_t kMaxTicketMaps = 256;
 
 struct TicketMap {
-  // classes present in the set: (dim, p1, fm), first ticket-map entry, count
-  struct Cls { int dim, p1, fm, lpc; long first, count; };
+  // classes present in the set: (dim, p1, fm, form), first ticket-map entry, count
+  struct Cls { int dim, p1, fm, lpc; bool grouped; long first, count; };
   std::vector<Cls> cls;
   DevBuf d;  // int2 (problem, task) entries of all classes
 };
@@ -136,11 +136,14 @@ int ticket_map(ouranos_batch* b, const std::vector<char>& mask, TicketMap** out)
     if (!mask[p] || done[p]) continue;
     const ouranos_rt* r = b->rt[p];
     const int dim = r->dim, p1 = r->p1, fm = b->fm[p], lpc = r->lpc;
+    const bool grouped = r->grouped;
     struct Key { double f; int p, t; };
     std::vector<Key> keys;
     for (size_t q = p; q < b->rt.size(); ++q) {
       const ouranos_rt* s = b->rt[q];
-      if (!mask[q] || done[q] || s->dim != dim || s->p1 != p1 || b->fm[q] != fm || s->lpc != lpc) continue;
+      if (!mask[q] || done[q] || s->dim != dim || s->p1 != p1 || b->fm[q] != fm || s->lpc != lpc ||
+          s->grouped != grouped)
+        continue;
       done[q] = 1;
       for (int t = 0; t < s->n_tasks; ++t) keys.push_back({(double)t / s->n_tasks, (int)q, t});
     }
@@ -148,7 +151,7 @@ int ticket_map(ouranos_batch* b, const std::vector<char>& mask, TicketMap** out)
       return x.f != y.f ? x.f < y.f : (x.p != y.p ? x.p < y.p : x.t < y.t);
     });
     if ((int)tm.cls.size() == kMaxClasses) return bbad(b, "too many problem classes in one batch");
-    tm.cls.push_back({dim, p1, fm, lpc, (long)all.size(), (long)keys.size()});
+    tm.cls.push_back({dim, p1, fm, lpc, grouped, (long)all.size(), (long)keys.size()});
     for (const Key& k : keys) all.push_back(make_int2(k.p, k.t));
   }
   BC(tm.d.alloc(sizeof(int2) * std::max<size_t>(all.size(), 1)), "ticket map");
@@ -191,7 +194,7 @@ int apply_body(ouranos_batch* b, const std::vector<char>& mask, bool sources, Ti
   for (size_t c = 0; c < tm->cls.size(); ++c) {
     const TicketMap::Cls& k = tm->cls[c];
     const int grid = (int)std::min<long>((k.count + 3) / 4, (long)std::max(1, b->sms * 8));
-    BC(launch_sweep_batch<real>(k.dim, k.p1, k.fm, k.lpc, d_args.as<SweepArgs<real>>(),
+    BC(launch_sweep_batch<real>(k.dim, k.p1, k.fm, k.lpc, k.grouped, sources, d_args.as<SweepArgs<real>>(),
                                 tm->d.as<int2>() + k.first, (int)k.count, ctrl + c, ctrl + kStatus,
                                 (const unsigned*)(ctrl + kEpoch), grid, 128, b->stream),
        "batched sweep");
@@ -348,13 +351,15 @@ int ouranos_batch_create(const ouranos_problem_desc* descs, int count, int devic
       return rc;
     }
     b->rt.push_back(r);
-    if (r->lpc == 32) {
+    if (!per_lane_order(r->dim, r->p1)) {
       char buf[256];
       std::snprintf(buf, sizeof buf,
                     "problem %d: the batched launch covers the per-lane sweep orders (2-D Q1..Q4, 3-D Q1..Q2)", p);
       b->err = buf;
       return OURANOS_ERR_UNSUPPORTED;
     }
+    r->in_batch = true;
+    BR(member(b, p, ouranos_rt_set_tiling(r, 0, 0, 0)));  // the default form of a batch's member
   }
   b->device = b->rt[0]->device;
   for (ouranos_rt* r : b->rt)
@@ -494,6 +499,7 @@ int ouranos_batch_autotune(ouranos_batch* b, int precision, int reps, int* tilin
       std::vector<std::vector<int>> cand;
       if (r->dim == 2) cand = {{32, 1, 1}, {16, 1, 2}, {8, 1, 4}, {4, 1, 8}};
       else cand = {{8, 4, 1}, {4, 4, 2}, {4, 2, 4}, {2, 2, 8}};
+      cand.push_back({0, 0, 0});  // the default form
       if (r->n >= 9) {  // two lanes per cell
         if (r->dim == 2) cand.insert(cand.end(), {{16, 1, 1}, {8, 1, 2}, {4, 1, 4}});
         else cand.insert(cand.end(), {{4, 4, 1}, {4, 2, 2}, {2, 2, 4}});
@@ -524,7 +530,7 @@ int ouranos_batch_autotune(ouranos_batch* b, int precision, int reps, int* tilin
     // problem sweeps timed above
     BR(member(b, (int)p, ouranos_rt_set_tiling(r, best[0], best[1], best[2])));
     if (tiling_out)
-      for (int k = 0; k < 3; ++k) tiling_out[3 * p + k] = best[k];
+      BR(member(b, (int)p, ouranos_rt_get_tiling(r, tiling_out + 3 * p, tiling_out + 3 * p + 1, tiling_out + 3 * p + 2)));
   }
   return size_buffers(b);
 }

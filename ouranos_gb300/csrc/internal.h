@@ -6,6 +6,7 @@
 #include <cmath>
 #include <cstdint>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/ouranos_gb300.h"
@@ -78,6 +79,13 @@ struct DevBuf {
   template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
+// the orders whose tilings name cells and directions per warp (2-D Q1..Q4, 3-D
+// Q1..Q2; every order, up to Q5, also runs one warp per cell), and those of them
+// with a per-lane kernel for each tiling (the others share a cell among lanes of
+// the library's choice)
+inline bool per_lane_order(int dim, int p1) { return dim == 2 ? p1 <= 5 : p1 <= 3; }
+inline bool per_lane_kernel(int dim, int p1) { return dim == 2 ? p1 <= 3 : p1 == 2; }
+
 // ---------------------------------------------------------- sweep kernels
 // Arguments of one sweep launch (see sweep.cuh for the algorithm).
 template <typename real>
@@ -114,7 +122,43 @@ struct SweepArgs {
   int wait_bias;
   int lpc;                     // lanes per cell: 1, 2 (cells of 9 or more dofs), or 32 (one warp
                                // per cell, sweep_wide.cuh; tiling 1 x 1 x 1, expanded source)
+  int grouped;                 // 1: the default form, lpc lanes per cell (sweep_group.cuh)
+  float minus_zero;            // -0, an addend the compiler does not know (pack2.cuh)
+  // one lane per cell (sweep_lane.cuh): the materials of the columns, four planes
+  // to a word, [sweep direction][plane / 4][column] (NULL: more than 256
+  // classes), and pairs of face-mass entries
+  const unsigned* cls4;
+  alignas(16) real facep[48];
+  const real* face_group;      // pairs of face-mass entries of the grouped form
 };
+
+// Pairs of face-mass entries of the one-lane-per-cell sweep (sweep_lane.cuh): in
+// 2-D [t][u] = (F_x, F_y), in 3-D [x, z, y][m][u] = rows (2m, 2m + 1) of the face
+template <typename real>
+void fill_face_pairs(const FETables& fe, real* out) {
+  const int fd = fe.fd;
+  if ((fe.dim == 2 && fd > 3) || (fe.dim == 3 && fd > 4)) return;  // (other forms)
+  auto F = [&](int ax, int t, int u) { return fe.face_mass[((size_t)ax * fd + t) * fd + u]; };
+  auto put = [&](int n, double v0, double v1) {
+    if constexpr (std::is_same<real, df64>::value) {
+      const df64 w0 = df64_split(v0), w1 = df64_split(v1);
+      out[2 * n] = df64(w0.hi, w1.hi);
+      out[2 * n + 1] = df64(w0.lo, w1.lo);
+    } else {
+      out[2 * n] = (real)v0;
+      out[2 * n + 1] = (real)v1;
+    }
+  };
+  int n = 0;
+  if (fe.dim == 2) {
+    for (int t = 0; t < fd; ++t)
+      for (int u = 0; u < fd; ++u) put(n++, F(0, t, u), F(1, t, u));
+  } else {
+    for (int ax : {0, 2, 1})
+      for (int m = 0; m < fd / 2; ++m)
+        for (int u = 0; u < fd; ++u) put(n++, F(ax, 2 * m, u), F(ax, 2 * m + 1, u));
+  }
+}
 
 // fused_moments: 0 = read the expanded per-direction source q; 1 or 2 = apply
 // M2D to that many source moments inside the sweep.
@@ -125,11 +169,22 @@ cudaError_t launch_sweep(int dim, int p1, int fused_moments, const SweepArgs<rea
 // of the orders the per-lane kernels do not instantiate (sweep_wide.cuh)
 template <typename real>
 cudaError_t launch_sweep_wide(int dim, int p1, const SweepArgs<real>& a, int grid, int block, cudaStream_t s);
+// one lane per cell, 2-D Q1 and Q2, 3-D Q1 (a.grouped, lpc 1; sweep_lane.cuh)
+template <typename real, int DIM>
+cudaError_t launch_sweep_lane(int p1, int fm, const SweepArgs<real>& a, int grid, int block, cudaStream_t s);
+// lpc lanes per cell through shared memory (a.grouped; sweep_group.cuh)
+template <typename real, int DIM>
+cudaError_t launch_sweep_group(int p1, int fm, const SweepArgs<real>& a, int grid, int block, cudaStream_t s);
+// the same two forms for a batch
+template <typename real, int DIM>
+cudaError_t launch_sweep_form_batch(int p1, int fm, int lpc, bool sources, const SweepArgs<real>* args, const int2* tmap,
+                                    int n_total, int* ticket, const int* status, const unsigned* epoch, int grid,
+                                    int block, cudaStream_t s);
 // Many problems in one persistent launch: args[p] per problem, tmap[t] =
 // (problem, task) for ticket t, epoch read from the device (all problems of
 // the launch share it), ticket reset to 0 by the caller.
 template <typename real>
-cudaError_t launch_sweep_batch(int dim, int p1, int fused_moments, int lanes_per_cell,
+cudaError_t launch_sweep_batch(int dim, int p1, int fused_moments, int lanes_per_cell, bool grouped, bool sources,
                                const SweepArgs<real>* args, const int2* tmap, int n_total, int* ticket,
                                const int* status, const unsigned* epoch, int grid, int block, cudaStream_t s);
 // q[d][e] = sum_m M2D[d][m] T[m][e] (+ iso[e])  -- moment -> direction expansion.
@@ -337,6 +392,10 @@ int rt_apply_device(ouranos_rt* rt, const double* x, double* y);
 // allocation-free Apply (noalloc.cu): resolve its scratch array on `device`,
 // which must be current; once per device, called by ouranos_rt_create
 int noalloc_setup(int device);
+void nominal_tiling(const ouranos_rt* rt, int& wx, int& wy, int& lpc);
+// whether the default form may take warp tiles of wx x wy cells for values of
+// real_bytes: its scratch then holds the problem if the nominal tiling's did
+bool noalloc_fits(const ouranos_rt* rt, int wx, int wy, size_t real_bytes);
 int rt_rhs_device(ouranos_rt* rt, const double* gf, double* rhs);
 int rt_check_status(ouranos_rt* rt);
 // batched Apply pieces (see operator.cu)
@@ -396,7 +455,10 @@ struct ouranos_rt {
   ouranos::DevBuf d_oz_m2d, d_oz_d2m, d_oz_m2d_exp, d_oz_d2m_exp;
   // schedule
   int wx = 0, wy = 1, kd = 0;          // 0 = not chosen yet
-  int lpc = 1;                         // lanes per cell (2 only for cells of >= 9 dofs)
+  int tiling[3] = {0, 0, 1};           // the tiling set by the caller (0: the default)
+  int lpc = 1;                         // lanes per cell
+  bool in_batch = false;               // a member of a batch (default_tiling)
+  bool grouped = false;                // the default form (sweep_group.cuh); wx, wy, lpc are its own
   int tiles_x = 0, tiles_y = 0, n_groups_dir = 0, n_tasks = 0;
   std::vector<int> dir_class_h;
   std::vector<double> class_abs_omega;  // [n_dir_class][3]
@@ -411,6 +473,8 @@ struct ouranos_rt {
   bool ainv_valid = false;
   bool scat_valid = false;             // src_* holds compute_scattering_source(x)
   // device: geometry / tables (both precisions where the sweep reads them)
+  ouranos::DevBuf d_cls4, d_fgroup64, d_fgroup32, d_fgroupdf;
+  bool cls4_ok = false;
   ouranos::DevBuf d_material, d_source_id, d_cell_class, d_cell_order;
   ouranos::DevBuf d_cell_mass, d_rowsum_mass, d_sscale, d_oscale, d_qcell;
   ouranos::DevBuf d_dir_class, d_abs64, d_abs32, d_m2d64, d_m2d32, d_d2m64, d_d2m32;

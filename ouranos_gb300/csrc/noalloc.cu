@@ -73,10 +73,12 @@ struct Layout {
   size_t edge_x_bytes, edge_y_bytes;
 };
 
-Layout layout_for(const ouranos_rt* rt, size_t real_bytes, bool expand) {
+// with warp tiles of wx x wy cells; word_bytes: bytes of an edge value's tagged words
+Layout layout_for(const ouranos_rt* rt, int wx, int wy, size_t real_bytes, size_t word_bytes, bool expand) {
   Layout L;
   const size_t nd = rt->n_dofs;
-  const size_t tiles = (size_t)rt->tiles_x * rt->tiles_y;
+  const size_t NX = rt->nx[0], NY = rt->dim == 3 ? rt->nx[1] : 1;
+  const size_t tiles = (NX + wx - 1) / wx * (rt->dim == 3 ? (NY + wy - 1) / wy : 1);
   const size_t NS = rt->nx[rt->dim - 1];
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -89,9 +91,8 @@ Layout layout_for(const ouranos_rt* rt, size_t real_bytes, bool expand) {
   L.q = expand ? take(real_bytes * rt->n_dir * nd) : 0;
   L.psi = take(real_bytes * rt->n_dir * nd);
   L.phi = take(real_bytes * rt->n_mom * nd);
-  // two tagged 64-bit words per edge value cover both precisions
-  L.edge_x_bytes = 16 * (size_t)rt->n_dir * tiles * NS * rt->wy * rt->fd;
-  L.edge_y_bytes = rt->dim == 3 ? 16 * (size_t)rt->n_dir * tiles * NS * rt->wx * rt->fd : 16;
+  L.edge_x_bytes = word_bytes * (size_t)rt->n_dir * tiles * NS * wy * rt->fd;
+  L.edge_y_bytes = rt->dim == 3 ? word_bytes * (size_t)rt->n_dir * tiles * NS * wx * rt->fd : 16;
   L.edge_x = take(L.edge_x_bytes);
   L.edge_y = take(L.edge_y_bytes);
   const bool perm = !rt->cell_order.empty();
@@ -99,6 +100,20 @@ Layout layout_for(const ouranos_rt* rt, size_t real_bytes, bool expand) {
   L.yout = perm ? take(8 * (size_t)rt->n_mom * nd) : 0;
   L.total = off;
   return L;
+}
+
+// the source is expanded, as in the regular Apply, when it has more moments than
+// the sweep applies in place (one warp per cell always reads it expanded)
+bool expands(const ouranos_rt* rt, bool wide) {
+  return !(rt->n_mom <= 2 && rt->n * (rt->n_mom + 1) <= 32) || wide;
+}
+
+// scratch of the problem with the nominal tiling, two tagged 64-bit words to an
+// edge value of either precision
+size_t nominal_bytes(const ouranos_rt* rt, size_t real_bytes) {
+  int wx = 0, wy = 0, lpc = 0;
+  nominal_tiling(rt, wx, wy, lpc);
+  return layout_for(rt, wx, wy, real_bytes, 16, expands(rt, lpc == 32)).total;
 }
 
 // the table of the sweep's arithmetic type (as the regular Apply reads them)
@@ -193,6 +208,11 @@ int apply_noalloc(ouranos_rt* rt, unsigned char* base, const Layout& L, bool exp
   a.wy = rt->wy;
   a.kd = rt->kd;
   a.lpc = rt->lpc;
+  a.grouped = rt->grouped;
+  a.cls4 = rt->cls4_ok ? rt->d_cls4.as<unsigned>() : nullptr;
+  a.face_group = tbl<real>(rt->d_fgroup64, rt->d_fgroup32, rt->d_fgroupdf);
+  a.minus_zero = -0.f;
+  fill_face_pairs(rt->fe, a.facep);
   a.tiles_x = rt->tiles_x;
   a.tiles_y = rt->tiles_y;
   a.n_tasks = rt->n_tasks;
@@ -255,6 +275,10 @@ int noalloc_setup(int device) {
   g_scratch_ptr[device] = p;
   return OURANOS_OK;
 }
+bool noalloc_fits(const ouranos_rt* rt, int wx, int wy, size_t real_bytes) {
+  return nominal_bytes(rt, real_bytes) > kNoAllocScratchBytes ||
+         layout_for(rt, wx, wy, real_bytes, 2 * real_bytes, expands(rt, false)).total <= kNoAllocScratchBytes;
+}
 }  // namespace ouranos
 
 extern "C" int ouranos_rt_apply_noalloc(ouranos_rt* rt, const double* x, double* y) {
@@ -263,18 +287,20 @@ extern "C" int ouranos_rt_apply_noalloc(ouranos_rt* rt, const double* x, double*
   if (!on_device(x) || !on_device(y))
     return fail(rt, OURANOS_ERR_BAD_INPUT,
                 "ouranos_rt_apply_noalloc takes device pointers only (no staging buffers)");
-  // same form choice as the regular Apply: expand the source when it has more
-  // moments than the sweep applies in place
-  const bool expand_source = !(rt->n_mom <= 2 && rt->n * (rt->n_mom + 1) <= 32) || rt->lpc == 32;
+  const bool expand_source = expands(rt, rt->lpc == 32 && !rt->grouped);
   // double, and the double-float pairs, take 8 bytes a value
   const size_t rb = rt->precision == OURANOS_FP64 ? 8 : 4;
-  const Layout L = layout_for(rt, rb, expand_source);
-  if (L.total > kNoAllocScratchBytes) {
+  const Layout L = layout_for(rt, rt->wx, rt->wy, rb, 2 * rb, expand_source);
+  // what it takes is counted with the nominal tiling; the default form is only
+  // chosen where it needs no more room than there is (noalloc_fits)
+  const size_t nominal = nominal_bytes(rt, rb);
+  const size_t need = rt->grouped ? std::max(nominal, L.total) : L.total;
+  if (need > kNoAllocScratchBytes) {
     char buf[256];
     std::snprintf(buf, sizeof buf,
                   "problem needs %zu bytes of scratch; the allocation-free Apply holds at most %zu "
                   "(use ouranos_rt_apply)",
-                  L.total, kNoAllocScratchBytes);
+                  need, kNoAllocScratchBytes);
     return fail(rt, OURANOS_ERR_BAD_INPUT, buf);
   }
   if (rt->device < 0 || rt->device >= kMaxDevices)

@@ -16,6 +16,10 @@ using namespace ouranos;
 
 namespace {
 
+// the sweep streams its sources in aligned 16-byte pieces, the last of which may
+// reach past the last value: every source buffer is this much longer
+constexpr size_t kSrcSlack = 16;
+
 #define OK_OR_RETURN(expr)                 \
   do {                                     \
     int _rc = (expr);                      \
@@ -244,31 +248,161 @@ int build_schedule(ouranos_rt* rt) {
   return OURANOS_OK;
 }
 
-// the per-lane sweep kernels are instantiated for 2-D Q1..Q4 and 3-D Q1..Q2;
-// every order (up to Q5) also runs one warp per cell
-static bool register_form(const ouranos_rt* rt) { return rt->dim == 2 ? rt->p1 <= 5 : rt->p1 <= 3; }
+// bytes of the edge buffers (build_schedule)
+size_t edge_bytes(const ouranos_rt* rt, int wx, int wy) {
+  const size_t NX = rt->nx[0], NY = rt->dim == 3 ? rt->nx[1] : 1, NS = rt->nx[rt->dim - 1];
+  const size_t tiles = ((NX + wx - 1) / wx) * (rt->dim == 3 ? (NY + wy - 1) / wy : 1);
+  return 16 * (size_t)rt->n_dir * tiles * NS * rt->fd * (rt->dim == 3 ? wx + wy : wy);
+}
 
+// The default sweep: lpc lanes to a cell of the grouped forms (1: sweep_lane.cuh,
+// else sweep_group.cuh), by what the cell needs and how many warps the problem
+// brings.  Sweep kernel on GB300, double-float / FP32, us; "nominal" is the per-lane
+// or one-warp-per-cell form of the nominal tiling, which was the default before:
+//   2-D Q1 256^2 LS S16    nominal 563 / 385     1 lane  438 / 276
+//   2-D Q2 256^2 LS S16    nominal 1144 / 769    1 lane  1098 / 500   4 lanes 1220 / 577
+//   2-D Q2 100^2 LS S8     nominal 292 / 221     1 lane  305 / 176    4 lanes 278 / 174
+//   2-D Q2 40^2 LS S8      nominal 126 / 83      1 lane  139 / 82     4 lanes 108 / 72
+//   2-D Q3 135x93 LS S12   nominal 849 / 352     4 lanes 532 / 217    8 lanes 430 / 231
+//   2-D Q4 200^2 LS S12    nominal 6734 / 2982   4 lanes 2356 / 879   8 lanes 2171 / 862
+//   2-D Q5 64^2 LS S8      nominal 972 / 518     8 lanes 884 / 198    16 lanes 606 / 207
+//   3-D Q1 64^3 GLC S12    nominal 4533 / 1863   1 lane  3381 / 1261  2 lanes 4953 / 1933
+//   3-D Q2 48^3 LS S8      nominal 17419 / 7391  8 lanes 6542 / 2193  16 lanes 6560 / 2740
+//   3-D Q2 16^3 LS S4      nominal 933 / 358     8 lanes 245 / 124    16 lanes 202 / 79
+//   3-D Q3 32^3 LS S8      nominal 11977 / 5784  8 lanes 11859 / 2470 16 lanes 7469 / 2336
+//   3-D Q4 10^3 LS S4      nominal 1020 / 448    16 lanes 959 / 414   32 lanes 579 / 280
+//   3-D Q5 8^3 LS S4       nominal 2682 / 1208   32 lanes 969 / 369
+// More lanes to a cell shorten a step (small problems wait on the wavefront's
+// steps), fewer spend less of it on passing b and the faces around.  A member of a
+// batch counts as a large problem: the batch's launch is full anyway, and fewer
+// forms are fewer launches.  Two lanes to a cell have the nominal tiling's tiles:
+// the last resort of the orders without a per-lane kernel.
 int default_tiling(ouranos_rt* rt) {
-  // one direction per warp: every lane of a warp reads the same inverse table
-  // (broadcast loads); 32 cells per warp (2-D: 32 x 1, 3-D: 4 x 8), or 16
-  // cells solved by two lanes each for cells of 9 or more dofs (3-D: 4 x 4).
-  // Measured on GB300, 64^3 Q1 GLC S12 FP32 sweep: 4 x 8 1.80 ms, 8 x 4 1.86,
-  // 4 x 4 x 2 directions 1.94, 8 x 2 x 2 2.21.  Higher orders: one warp per cell.
   rt->kd = 1;
-  if (!register_form(rt)) {
-    rt->wx = rt->wy = 1;
-    rt->lpc = 32;
+  int wx0 = 0, wy0 = 0, lpc0 = 0;
+  nominal_tiling(rt, wx0, wy0, lpc0);
+  const long tiles_x = (rt->nx[0] + 31) / 32, tiles_2 = (long)((rt->nx[0] + 1) / 2) * ((rt->nx[1] + 1) / 2);
+  std::vector<int> lanes;
+  if (rt->dim == 2) {
+    switch (rt->p1) {
+      case 2: lanes = {1}; break;
+      case 3: lanes = rt->n_dir * tiles_x < 256 && !rt->in_batch ? std::vector<int>{4, 1} : std::vector<int>{1}; break;
+      case 4: case 5: lanes = {8, 2}; break;
+      default: lanes = {16}; break;
+    }
+  } else {
+    switch (rt->p1) {
+      case 2: lanes = {1}; break;
+      case 3: lanes = rt->n_dir * tiles_2 < 4096 && !rt->in_batch ? std::vector<int>{16, 8, 2} : std::vector<int>{8, 2}; break;
+      case 4: lanes = {16}; break;
+      default: lanes = {32}; break;
+    }
+  }
+  if (rt->n_mom == 2 && rt->n * 3 <= 32) lanes.clear();  // two fused moments: the per-lane form
+  // one lane per cell counts dofs in an int (also of the planes the tile's skew
+  // walks in from)
+  const long plane = rt->n_cells / rt->nx[rt->dim - 1];
+  const bool wide_index = rt->n * (rt->n_cells + 40 * plane) >= (1L << 31);
+  size_t free_b = 0, total_b = 0;
+  CU(cudaMemGetInfo(&free_b, &total_b), "device memory");
+  for (int H : lanes) {
+    const int G = 32 / H;
+    const int wx = rt->dim == 2 ? G : (G >= 8 ? 4 : (G >= 2 ? 2 : 1)), wy = G / wx;
+    if (H == 1 && wide_index) continue;
+    // smaller tiles hand over more edges: not where these crowd out the angular
+    // flux and the expanded source, nor where the allocation-free Apply would no
+    // longer hold a problem it holds with the nominal tiling
+    if (H != 2 && edge_bytes(rt, wx, wy) > edge_bytes(rt, wx0, wy0) &&
+        edge_bytes(rt, wx, wy) + 16 * (size_t)rt->n_dir * rt->n_dofs > free_b / 2)
+      continue;
+    bool fits = true;
+    for (size_t rb : {4, 8}) fits = fits && noalloc_fits(rt, wx, wy, rb);
+    if (!fits && H != 2) continue;
+    rt->wx = wx;
+    rt->wy = wy;
+    rt->lpc = H;
+    rt->grouped = true;
     return OURANOS_OK;
   }
-  rt->lpc = rt->n >= 9 ? 2 : 1;
-  if (rt->dim == 2) {
-    rt->wx = 32 / rt->lpc;
-    rt->wy = 1;
-  } else {
-    rt->wx = 4;
-    rt->wy = rt->lpc == 2 ? 4 : 8;
-  }
+  rt->wx = wx0;
+  rt->wy = wy0;
+  rt->lpc = lpc0;
+  rt->grouped = false;
   return OURANOS_OK;
+}
+
+// The inverse tables of the grouped sweep (layout: GroupRows in
+// sweep_group.cuh): per matrix the row pairs, [pair][16-byte piece of columns]
+// [lane], each column {v0, v1} (double-float: {hi0, hi1, lo0, lo1}), then the
+// lone rows, [16-byte piece of columns][lane]; the rest is zero
+template <typename real>
+std::vector<unsigned char> group_tables(const std::vector<double>& ainv, size_t mats, int dim, int p1, int H) {
+  const int n = dim == 2 ? p1 * p1 : p1 * p1 * p1, sz = (int)sizeof(real);
+  const bool adj = p1 % 2 == 0 && (n / 2) % H == 0;
+  const int R = (n + H - 1) / H, RP = R / 2;
+  const int pj = 8 / sz, ncp = (n + pj - 1) / pj, pl = 16 / sz, ncl = R % 2 ? (n + pl - 1) / pl : 0;
+  const size_t bytes = (size_t)16 * H * (RP * ncp + ncl);
+  std::vector<unsigned char> out(mats * bytes, 0);
+  for (size_t m = 0; m < mats; ++m)
+    for (int h = 0; h < H; ++h)
+      for (int k = 0; k < R; ++k) {
+        const int i = adj ? 2 * (h + H * (k / 2)) + k % 2 : h + H * k;
+        if (i >= n) continue;
+        for (int j = 0; j < n; ++j) {
+          const double v = ainv[(m * n + i) * n + j];
+          unsigned char* at = out.data() + m * bytes;
+          const bool pair = k / 2 < RP;
+          if (pair) at += ((size_t)((k / 2) * ncp + j / pj) * H + h) * 16 + (j % pj) * 2 * sz;
+          else at += ((size_t)RP * ncp * H + (size_t)(j / pl) * H + h) * 16 + (j % pl) * sz;
+          if constexpr (std::is_same<real, df64>::value) {
+            const df64 w = df64_split(v);
+            std::memcpy(at + (pair ? 4 * (k % 2) : 0), &w.hi, 4);
+            std::memcpy(at + (pair ? 8 + 4 * (k % 2) : 4), &w.lo, 4);
+          } else {
+            const real w = (real)v;
+            std::memcpy(at + (pair ? sz * (k % 2) : 0), &w, sz);
+          }
+        }
+      }
+  return out;
+}
+
+// The face-mass rows of the grouped sweep, two at a time and H lanes side by side
+// ([row pair][column][lane], see GroupRows): the row pairs of every axis and, where
+// a face leaves each lane an odd number of rows, its last x row with its last y
+// row, then its last z row twice; rows past the last are zero
+template <typename real>
+std::vector<unsigned char> group_face_table(const FETables& fe, int H) {
+  const int fd = fe.fd, dim = fe.dim, sz = (int)sizeof(real);
+  const bool adj = fe.p1 % 2 == 0 && (fe.n / 2) % H == 0;
+  const int KF = adj ? 2 * ((fd / 2 + H - 1) / H) : (fd + H - 1) / H, FP = KF / 2;
+  const bool mix = !adj && KF % 2 != 0;
+  const int nfr = dim * FP + (mix ? dim - 1 : 0);
+  std::vector<unsigned char> out((size_t)nfr * fd * H * 2 * sz, 0);
+  auto F = [&](int ax, int t, int u) { return t < fd ? fe.face_mass[((size_t)ax * fd + t) * fd + u] : 0.0; };
+  for (int n = 0; n < nfr; ++n)
+    for (int u = 0; u < fd; ++u)
+      for (int h = 0; h < H; ++h) {
+        auto row = [&](int k) { return adj ? 2 * (h + H * (k / 2)) + k % 2 : h + H * k; };
+        double v[2];
+        if (n < dim * FP) {
+          for (int r = 0; r < 2; ++r) v[r] = F(n / FP, row(2 * (n % FP) + r), u);
+        } else {
+          for (int r = 0; r < 2; ++r) v[r] = F(n == dim * FP ? r : 2, row(KF - 1), u);
+        }
+        unsigned char* at = out.data() + (((size_t)n * fd + u) * H + h) * 2 * sz;
+        for (int r = 0; r < 2; ++r) {
+          if constexpr (std::is_same<real, df64>::value) {
+            const df64 w = df64_split(v[r]);
+            std::memcpy(at + 4 * r, &w.hi, 4);
+            std::memcpy(at + 8 + 4 * r, &w.lo, 4);
+          } else {
+            const real w = (real)v[r];
+            std::memcpy(at + sz * r, &w, sz);
+          }
+        }
+      }
+  return out;
 }
 
 // ------------------------------------------------------- per-group tables
@@ -292,6 +426,18 @@ int setup_group(ouranos_rt* rt) {
   std::vector<int> ccls(rt->n_cells);
   for (long c = 0; c < rt->n_cells; ++c) ccls[c] = mat_cls[rt->material_id[c]];
   OK_OR_RETURN(upload(rt, rt->d_cell_class, ccls, "cell classes"));
+  // the columns' classes, four planes to a word, for either sweep direction
+  rt->cls4_ok = rt->grouped && rt->lpc == 1 && cls_val.size() <= 256;
+  if (rt->cls4_ok) {
+    const long NS = rt->nx[rt->dim - 1], ncol = rt->n_cells / NS, words = (NS + 3) / 4;
+    std::vector<unsigned> packed((size_t)2 * words * ncol, 0u);
+    for (int dir = 0; dir < 2; ++dir)
+      for (long k = 0; k < NS; ++k)
+        for (long c = 0; c < ncol; ++c)
+          packed[((size_t)dir * words + k / 4) * ncol + c] |=
+              (unsigned)ccls[c + ncol * (dir ? NS - 1 - k : k)] << (8 * (k % 4));
+    OK_OR_RETURN(upload(rt, rt->d_cls4, packed, "cell classes"));
+  }
   // A'^-1 per (sigma class, |Omega| class)
   const size_t nn = (size_t)n * n;
   std::vector<double> ainv(cls_val.size() * rt->n_dir_class * nn);
@@ -303,7 +449,17 @@ int setup_group(ouranos_rt* rt) {
   // loads them as vectors); one warp per cell reads the transpose, whose row j
   // holds entry (i, j) for consecutive i
   std::vector<double> ainv_p;
-  if (rt->lpc == 32) {
+  if (rt->grouped) {
+    const size_t mats = cls_val.size() * rt->n_dir_class;
+    if (rt->lpc > 1) {
+      OK_OR_RETURN(upload(rt, rt->d_fgroup64, group_face_table<double>(rt->fe, rt->lpc), "face tables"));
+      OK_OR_RETURN(upload(rt, rt->d_fgroupdf, group_face_table<df64>(rt->fe, rt->lpc), "face tables"));
+      OK_OR_RETURN(upload(rt, rt->d_fgroup32, group_face_table<float>(rt->fe, rt->lpc), "face tables"));
+    }
+    OK_OR_RETURN(upload(rt, rt->d_ainv64, group_tables<double>(ainv, mats, rt->dim, rt->p1, rt->lpc), "inverse tables"));
+    OK_OR_RETURN(upload(rt, rt->d_ainvdf, group_tables<df64>(ainv, mats, rt->dim, rt->p1, rt->lpc), "inverse tables"));
+    OK_OR_RETURN(upload(rt, rt->d_ainv32, group_tables<float>(ainv, mats, rt->dim, rt->p1, rt->lpc), "inverse tables"));
+  } else if (rt->lpc == 32) {
     ainv_p.resize(ainv.size());
     const size_t mats = cls_val.size() * rt->n_dir_class;
     for (size_t m = 0; m < mats; ++m)
@@ -312,9 +468,11 @@ int setup_group(ouranos_rt* rt) {
   } else {
     ainv_p = pad_rows(ainv, (long)cls_val.size() * rt->n_dir_class * n, n);
   }
-  OK_OR_RETURN(upload(rt, rt->d_ainv64, ainv_p, "inverse tables"));
-  OK_OR_RETURN(upload(rt, rt->d_ainv32, to_f32(ainv_p), "inverse tables"));
-  OK_OR_RETURN(upload(rt, rt->d_ainvdf, to_df(ainv_p), "inverse tables"));
+  if (!rt->grouped) {
+    OK_OR_RETURN(upload(rt, rt->d_ainv64, ainv_p, "inverse tables"));
+    OK_OR_RETURN(upload(rt, rt->d_ainv32, to_f32(ainv_p), "inverse tables"));
+    OK_OR_RETURN(upload(rt, rt->d_ainvdf, to_df(ainv_p), "inverse tables"));
+  }
   // scattering scales: sigma_s(mat, g'->g, l(m)) (by Legendre order)
   auto sig_s = [&](int mat, int gf, int gt, int l) {
     if (l > L) return 0.0;
@@ -409,6 +567,11 @@ int sweep_prepare(ouranos_rt* rt, const real* src, const real* iso, const real* 
   a.wy = rt->wy;
   a.kd = rt->kd;
   a.lpc = rt->lpc;
+  a.grouped = rt->grouped;
+  a.cls4 = rt->cls4_ok ? rt->d_cls4.as<unsigned>() : nullptr;
+  a.face_group = table<real>(rt->d_fgroup64, rt->d_fgroup32, rt->d_fgroupdf);
+  a.minus_zero = -0.f;
+  fill_face_pairs(rt->fe, a.facep);
   a.tiles_x = rt->tiles_x;
   a.tiles_y = rt->tiles_y;
   a.n_tasks = rt->n_tasks;
@@ -440,9 +603,9 @@ int sweep_prepare(ouranos_rt* rt, const real* src, const real* iso, const real* 
   fm = (rt->n_mom <= kFusedMomentsMax && rt->n * (rt->n_mom + 1) <= 32) ? rt->n_mom : 0;
   // a source sweep of a time step carries the per-direction psi^n term: expanded form
   const bool angular = iso && rt->inv_vdt > 0.0 && rt->d_psi_prev.p;
-  if (angular || rt->lpc == 32) fm = 0;  // (one warp per cell reads the expanded source only)
+  if (angular || (rt->lpc == 32 && !rt->grouped)) fm = 0;  // (one warp per cell reads the expanded source only)
   if (fm == 0) {
-    CU(rt->d_q.alloc(sizeof(real) * len_dir), "expanded source");
+    CU(rt->d_q.alloc(sizeof(real) * len_dir + kSrcSlack), "expanded source");
     a.q = rt->d_q.as<real>();
     if (expand) {
       OK_OR_RETURN(sweep_expand<real>(rt, src, iso, 0, rt->n_dofs));
@@ -649,19 +812,19 @@ int build_source(ouranos_rt* rt, const double* x, const double* gf, bool pairs, 
   if (gf) gf += o;
   const int* mat = rt->d_material.as<int>() + c0;
   if (rt->precision == OURANOS_FP64 && pairs) {
-    CU(rt->d_src64.alloc(sizeof(df64) * len), "source");
+    CU(rt->d_src64.alloc(sizeof(df64) * len + kSrcSlack), "source");
     CU(launch_scatter_source<df64>(x, gf, rt->d_src64.as<df64>() + o, M, rt->d_sscale.as<double>(),
                                    rt->d_oscale.as<double>(), mat, rt->n_mat, rt->G, rt->group, nc, rt->n,
                                    rt->n_mom, rt->n_dofs, rt->stream),
        "scattering source");
   } else if (rt->precision == OURANOS_FP64) {
-    CU(rt->d_src64.alloc(sizeof(double) * len), "source");
+    CU(rt->d_src64.alloc(sizeof(double) * len + kSrcSlack), "source");
     CU(launch_scatter_source<double>(x, gf, rt->d_src64.as<double>() + o, M, rt->d_sscale.as<double>(),
                                      rt->d_oscale.as<double>(), mat, rt->n_mat, rt->G, rt->group, nc, rt->n,
                                      rt->n_mom, rt->n_dofs, rt->stream),
        "scattering source");
   } else {
-    CU(rt->d_src32.alloc(sizeof(float) * len), "source");
+    CU(rt->d_src32.alloc(sizeof(float) * len + kSrcSlack), "source");
     CU(launch_scatter_source<float>(x, gf, rt->d_src32.as<float>() + o, M, rt->d_sscale.as<double>(),
                                     rt->d_oscale.as<double>(), mat, rt->n_mat, rt->G, rt->group, nc, rt->n,
                                     rt->n_mom, rt->n_dofs, rt->stream),
@@ -677,7 +840,7 @@ int sweep_into_phi(ouranos_rt* rt, bool sources) {
     CU(rt->d_phi64.alloc(sizeof(double) * len), "flux");
     const df64* iso = nullptr;
     if (sources) {
-      CU(rt->d_iso64.alloc(sizeof(df64) * rt->n_dofs), "iso");
+      CU(rt->d_iso64.alloc(sizeof(df64) * rt->n_dofs + kSrcSlack), "iso");
       CU(launch_iso_source<df64>(rt->d_iso64.as<df64>(), rt->d_qcell.as<double>(),
                                  rt->d_rowsum_mass.as<double>(), rt->d_source_id.as<int>(), rt->n_cells,
                                  rt->n, rt->stream),
@@ -691,7 +854,7 @@ int sweep_into_phi(ouranos_rt* rt, bool sources) {
     CU(rt->d_phi64.alloc(sizeof(double) * len), "flux");
     const double* iso = nullptr;
     if (sources) {
-      CU(rt->d_iso64.alloc(sizeof(double) * rt->n_dofs), "iso");
+      CU(rt->d_iso64.alloc(sizeof(double) * rt->n_dofs + kSrcSlack), "iso");
       CU(launch_iso_source<double>(rt->d_iso64.as<double>(), rt->d_qcell.as<double>(),
                                    rt->d_rowsum_mass.as<double>(), rt->d_source_id.as<int>(),
                                    rt->n_cells, rt->n, rt->stream),
@@ -704,7 +867,7 @@ int sweep_into_phi(ouranos_rt* rt, bool sources) {
   CU(rt->d_phi32.alloc(sizeof(float) * len), "flux");
   const float* iso = nullptr;
   if (sources) {
-    CU(rt->d_iso32.alloc(sizeof(float) * rt->n_dofs), "iso");
+    CU(rt->d_iso32.alloc(sizeof(float) * rt->n_dofs + kSrcSlack), "iso");
     CU(launch_iso_source<float>(rt->d_iso32.as<float>(), rt->d_qcell.as<double>(),
                                 rt->d_rowsum_mass.as<double>(), rt->d_source_id.as<int>(),
                                 rt->n_cells, rt->n, rt->stream),
@@ -743,7 +906,7 @@ int apply_overlapped(ouranos_rt* rt, const double* hx, double* hy) {
   CU(rt->d_x.alloc(sizeof(double) * len), "staging");
   CU(rt->d_y.alloc(sizeof(double) * len), "apply");
   DevBuf& sb = f64 ? rt->d_src64 : rt->d_src32;
-  CU(sb.alloc(sizeof(real) * len), "source");
+  CU(sb.alloc(sizeof(real) * len + kSrcSlack), "source");
   DevBuf& pb = f64 ? rt->d_phi64 : rt->d_phi32;
   CU(pb.alloc((f64 ? sizeof(double) : sizeof(float)) * len), "flux");
   if (!rt->copy_stream) {
@@ -825,6 +988,21 @@ int apply_overlapped(ouranos_rt* rt, const double* hx, double* hy) {
 
 // ============================================================== internal API
 namespace ouranos {
+// The nominal default tiling, which ouranos_rt_get_tiling reports while no other
+// was set: one direction per warp, 32 cells per warp (2-D 32 x 1, 3-D 4 x 8), 16
+// for cells of 9 or more dofs (3-D 4 x 4), one for the orders above 2-D Q4 and
+// 3-D Q2
+void nominal_tiling(const ouranos_rt* rt, int& wx, int& wy, int& lpc) {
+  if (!per_lane_order(rt->dim, rt->p1)) {
+    wx = wy = 1;
+    lpc = 32;
+    return;
+  }
+  lpc = rt->n >= 9 ? 2 : 1;
+  wx = rt->dim == 2 ? 32 / lpc : 4;
+  wy = rt->dim == 2 ? 1 : (lpc == 2 ? 4 : 8);
+}
+
 // Device-side Apply for the solvers: y = x - D L^-1 M2D S x, x and y device,
 // lexicographic numbering.  Does not synchronise.
 int rt_apply_device(ouranos_rt* rt, const double* x, double* y) {
@@ -862,7 +1040,7 @@ static int batch_prepare(ouranos_rt* rt, const double* x, SweepArgs<real>* a, in
   const real* bnd = nullptr;
   if (sources) {
     DevBuf& ib = f64 ? rt->d_iso64 : rt->d_iso32;
-    CU(ib.alloc(sizeof(real) * rt->n_dofs), "iso");
+    CU(ib.alloc(sizeof(real) * rt->n_dofs + kSrcSlack), "iso");
     CU(launch_iso_source<real>(ib.as<real>(), rt->d_qcell.as<double>(), rt->d_rowsum_mass.as<double>(),
                                rt->d_source_id.as<int>(), rt->n_cells, rt->n, rt->stream),
        "iso source");
@@ -1376,9 +1554,13 @@ int ouranos_rt_last_sweep_ms(const ouranos_rt* rt, double* ms, int* kernels) {
 int ouranos_rt_set_tiling(ouranos_rt* rt, int cells_x, int cells_y, int dirs) {
   if (!rt) return OURANOS_ERR_BAD_INPUT;
   cudaSetDevice(rt->device);
-  const bool was_wide = rt->lpc == 32;
+  // the layout of the inverse tables: the grouped forms' by their lanes, the
+  // transposed one of one warp per cell, or rows
+  auto layout = [&] { return rt->grouped ? 100 + rt->lpc : (rt->lpc == 32 ? 32 : 0); };
+  const int before = layout();
   if (cells_x == 0 && cells_y == 0 && dirs == 0) {
     OK_OR_RETURN(default_tiling(rt));
+    rt->tiling[0] = 0;
   } else {
     if (rt->dim == 2) cells_y = 1;
     const int lanes = cells_x * cells_y * dirs;
@@ -1387,25 +1569,35 @@ int ouranos_rt_set_tiling(ouranos_rt* rt, int cells_x, int cells_y, int dirs) {
     if (cells_x < 1 || cells_y < 1 || dirs < 1 || (lanes != 32 && !two && !wide) || (dirs & (dirs - 1)))
       return bad(rt, "tiling must satisfy cells_x*cells_y*dirs == 32 (or 16, two lanes per cell, for cells "
                      "of 9 or more dofs; or 1 x 1 x 1, one warp per cell) with dirs a power of two");
-    if (!wide && !register_form(rt))
+    if (!wide && !per_lane_order(rt->dim, rt->p1))
       return bad(rt, "this DG order runs one warp per cell only (tiling 1 x 1 x 1): the per-lane sweep "
                      "covers 2-D Q1..Q4 and 3-D Q1..Q2");
-    rt->wx = cells_x;
-    rt->wy = cells_y;
-    rt->kd = dirs;
-    rt->lpc = wide ? 32 : (two ? 2 : 1);
+    if (!wide && !per_lane_kernel(rt->dim, rt->p1)) {
+      OK_OR_RETURN(default_tiling(rt));  // these orders' lanes share their cells whatever the tiling
+    } else {
+      rt->wx = cells_x;
+      rt->wy = cells_y;
+      rt->kd = dirs;
+      rt->lpc = wide ? 32 : (two ? 2 : 1);
+      rt->grouped = false;
+    }
+    rt->tiling[0] = cells_x;
+    rt->tiling[1] = cells_y;
+    rt->tiling[2] = dirs;
   }
   OK_OR_RETURN(build_schedule(rt));
-  if (was_wide != (rt->lpc == 32)) OK_OR_RETURN(setup_group(rt));  // the inverse tables change layout
+  if (layout() != before) OK_OR_RETURN(setup_group(rt));  // the tables change layout
   CU(cudaStreamSynchronize(rt->stream), "tiling");
   return OURANOS_OK;
 }
 
 int ouranos_rt_get_tiling(const ouranos_rt* rt, int* cx, int* cy, int* dirs) {
   if (!rt) return OURANOS_ERR_BAD_INPUT;
-  if (cx) *cx = rt->wx;
-  if (cy) *cy = rt->wy;
-  if (dirs) *dirs = rt->kd;
+  int wx = rt->tiling[0], wy = rt->tiling[1], lpc = 0;
+  if (!wx) nominal_tiling(rt, wx, wy, lpc);  // the default: its nominal tiling
+  if (cx) *cx = wx;
+  if (cy) *cy = wy;
+  if (dirs) *dirs = rt->tiling[0] ? rt->tiling[2] : 1;
   return OURANOS_OK;
 }
 

@@ -1,4 +1,6 @@
-// Transport sweep kernel for sm_103a.
+// Transport sweep kernel for sm_103a: the form with each cell in one lane's (or two
+// lanes') registers, run for the explicit tilings of 2-D Q1 and Q2 and 3-D Q1; the
+// default forms (sweep_lane.cuh, sweep_group.cuh) share its scheme and its bits.
 //
 // Replaces the reference's task loop
 //   initialize_scheduler(); while (n_tasks_to_execute) sweep(*get_next_task(), ...)
@@ -883,6 +885,32 @@ __global__ void __launch_bounds__(128) sweep_kernel(const SweepArgs<real> a) {
 // its task's problem arguments into its shared slot before the task; the
 // edge-word epoch comes from device memory, so a captured launch replays with
 // the epoch of the moment.
+template <typename real>
+__device__ __forceinline__ int next_batch_task(const SweepArgs<real>* __restrict__ args, const int2* __restrict__ tmap,
+                                               int n_total, int* ticket, const int* status, const unsigned* epoch,
+                                               SweepArgs<real>& slot) {
+  static_assert(sizeof(SweepArgs<real>) % 4 == 0, "argument block is copied by words");
+  constexpr int WORDS = (int)(sizeof(SweepArgs<real>) / 4);
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  int t = 0, stop = 0;
+  if (lane == 0) {
+    t = atomicAdd(ticket, 1);
+    stop = *(volatile const int*)status;
+  }
+  t = __shfl_sync(FULL, t, 0);
+  stop = __shfl_sync(FULL, stop, 0);
+  if (t >= n_total || stop) return -1;
+  const int2 pt = tmap[t];
+  const unsigned* src = reinterpret_cast<const unsigned*>(args + pt.x);
+  unsigned* dst = reinterpret_cast<unsigned*>(&slot);
+  for (int i = lane; i < WORDS; i += 32) dst[i] = src[i];
+  __syncwarp();
+  if (lane == 0) slot.epoch = *epoch;  // set on the device before the launch
+  __syncwarp();
+  return pt.y;
+}
+
 template <typename real, int DIM, int P1, int FM, int H>
 __global__ void __launch_bounds__(128) sweep_batch_kernel(const SweepArgs<real>* __restrict__ args,
                                                           const int2* __restrict__ tmap, int n_total,
@@ -890,28 +918,11 @@ __global__ void __launch_bounds__(128) sweep_batch_kernel(const SweepArgs<real>*
                                                           const unsigned* epoch) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ SweepArgs<real> s_args[4];
-  static_assert(sizeof(SweepArgs<real>) % 4 == 0, "argument block is copied by words");
-  constexpr int WORDS = (int)(sizeof(SweepArgs<real>) / 4);
-  constexpr unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   for (;;) {
-    int t = 0, stop = 0;
-    if (lane == 0) {
-      t = atomicAdd(ticket, 1);
-      stop = *(volatile const int*)status;
-    }
-    t = __shfl_sync(FULL, t, 0);
-    stop = __shfl_sync(FULL, stop, 0);
-    if (t >= n_total || stop) return;
-    const int2 pt = tmap[t];
-    const unsigned* src = reinterpret_cast<const unsigned*>(args + pt.x);
-    unsigned* dst = reinterpret_cast<unsigned*>(&s_args[warp]);
-    for (int i = lane; i < WORDS; i += 32) dst[i] = src[i];
-    __syncwarp();
-    if (lane == 0) s_args[warp].epoch = *epoch;  // set on the device before the launch
-    __syncwarp();
-    sweep_task<real, DIM, P1, FM, H>(s_args[warp], pt.y, smem_raw);
+    const int task = next_batch_task(args, tmap, n_total, ticket, status, epoch, s_args[warp]);
+    if (task < 0) return;
+    sweep_task<real, DIM, P1, FM, H>(s_args[warp], task, smem_raw);
     __syncwarp();  // the slot is rewritten by the next task
   }
 }

@@ -1,6 +1,6 @@
-// Instantiations of the sweep kernel in float: 2-D Q1..Q4, 3-D Q1..Q2
-// (one warp per cell for the 1 x 1 x 1 tiling and the higher orders:
-// sweep_wide_f32.cu).
+// Instantiations of the sweep kernel in float: the per-lane forms of the
+// explicit tilings, 2-D Q1 and Q2, 3-D Q1 (the default forms: sweep_lane_f32.cu,
+// sweep_group_f32_*.cu; one warp per cell: sweep_wide_f32.cu).
 #include "sweep.cuh"
 
 namespace ouranos {
@@ -8,18 +8,21 @@ namespace ouranos {
 template <>
 cudaError_t launch_sweep<float>(int dim, int p1, int fm, const SweepArgs<float>& a, int grid, int block,
                                 cudaStream_t s) {
+  if (a.grouped && a.lpc == 1)
+    return dim == 2 ? launch_sweep_lane<float, 2>(p1, fm, a, grid, block, s)
+                    : launch_sweep_lane<float, 3>(p1, fm, a, grid, block, s);
+  if (a.grouped)
+    return dim == 2 ? launch_sweep_group<float, 2>(p1, fm, a, grid, block, s)
+                    : launch_sweep_group<float, 3>(p1, fm, a, grid, block, s);
   if (a.lpc == 32) return launch_sweep_wide<float>(dim, p1, a, grid, block, s);
   if (dim == 2) {
     switch (p1) {
       case 2: return launch_sweep_impl<float, 2, 2>(fm, a, grid, block, s);
       case 3: return launch_sweep_impl<float, 2, 3>(fm, a, grid, block, s);
-      case 4: return launch_sweep_impl<float, 2, 4>(fm, a, grid, block, s);
-      case 5: return launch_sweep_impl<float, 2, 5>(fm, a, grid, block, s);
     }
   } else if (dim == 3) {
     switch (p1) {
       case 2: return launch_sweep_impl<float, 3, 2>(fm, a, grid, block, s);
-      case 3: return launch_sweep_impl<float, 3, 3>(fm, a, grid, block, s);
     }
   }
   return cudaErrorInvalidValue;
