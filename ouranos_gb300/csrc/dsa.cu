@@ -182,36 +182,8 @@ __device__ __forceinline__ void delta_nb(float (&nb)[3][3][3], int ex, int ey, i
       for (int dx = 0; dx < 3; ++dx) nb[dz][dy][dx] = (dx == ex && dy == ey && dz == ez) ? 1.f : 0.f;
 }
 
-// Fixed-order sum over a block of kCgThreads; thread 0 returns the total.
-__device__ __forceinline__ double block_sum(double t) {
-  __shared__ double red[kCgThreads / 32];
-  for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double u = red[threadIdx.x];
-    for (int o = 16; o; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
-    t = u;
-  }
-  __syncthreads();
-  return t;
-}
-
-// Sum of the nb per-block partials of a phase, in block order (every block
-// of the problem gets the same value).
-__device__ __forceinline__ double all_sum(const double* part, int nb) {
-  __shared__ double total;
-  double u = 0.0;
-  for (int i = threadIdx.x; i < nb; i += kCgThreads) u += part[i];
-  u = block_sum(u);
-  if (threadIdx.x == 0) total = u;
-  __syncthreads();
-  return total;
-}
-
 struct DsaSync {
-  unsigned count;  // blocks arrived at the current barrier
-  unsigned gen;    // barriers completed
+  unsigned count;  // arrivals at all barriers so far (zeroed before the launch)
 };
 constexpr int kStatusBarrier = 2;  // status bit: a barrier wait gave up
 
@@ -220,49 +192,133 @@ __device__ __forceinline__ unsigned long long global_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-__device__ __forceinline__ unsigned atom_add_acq_rel(unsigned* p, unsigned v) {
-  unsigned old;
-  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-  return old;
-}
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+__device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
   unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 
-// Grid-wide barrier of a cooperative launch (all blocks co-resident).
-// Thread 0 of each block arrives with a release (after the block's bar.sync)
-// and leaves with an acquire, so every write of any block before the barrier
-// is visible to every thread after it.  The wait is bounded by limit_ns: a
-// block that gives up sets the status bit and returns false, and blocks still
-// waiting elsewhere see the bit and give up too.  bias (a test hook) makes the
-// generation the waiters wait for one that never comes.  (Per-block epoch
-// words polled by every block, in place of the shared counter, measured
-// slower: 34.8 against 21.5 us per CG step at 152 blocks.)
-__device__ __forceinline__ bool grid_barrier(DsaSync* s, int* status, long long limit_ns, unsigned bias = 0) {
+// A grid-wide sum and barrier of a cooperative launch (all blocks co-resident).
+// Barrier: one counter that only grows; meeting number n (from 1) is over once
+// n gridDim.x blocks have arrived.  Thread 0 of each block arrives with a release
+// (after the block's bar.sync) and leaves with an acquire, so every write of any
+// block before the meeting is visible to every thread after it; the polls are
+// relaxed.  The wait is bounded by limit_ns: a block that gives up sets the status
+// bit and returns false, and blocks still waiting elsewhere see the bit and give up
+// too.  bias (a test hook) makes the waiters wait for an arrival that never comes.
+struct Meeting {
+  DsaSync* sync;
+  int* status;
+  long long limit_ns;
+  unsigned bias;
+  unsigned passed = 0;
+};
+
+// (t, e) += (o, oe): a float pair, Knuth's two-sum of the leading parts, some 48 bits
+__device__ __forceinline__ void pair_add(float& t, float& e, float o, float oe) {
+  const float s = __fadd_rn(t, o);
+  const float bb = __fsub_rn(s, t);
+  const float err = __fadd_rn(__fsub_rn(t, __fsub_rn(s, bb)), __fsub_rn(o, bb));
+  t = s;
+  e = __fadd_rn(__fadd_rn(e, oe), err);
+}
+
+__device__ __forceinline__ double warp_sum(double u) {
+  for (int o = 16; o; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
+  return u;
+}
+
+// sums[i] = the problem's sum of t[i] (its nb blocks, this one number lb, with a
+// partial each in part[i]); thread 0 turns the sums into one number, finish(sums),
+// which every thread returns in `result`.  A block adds its threads' FP32 values as
+// float pairs (exact sums with their errors kept), the block partials are FP64 and
+// added in block order by every block alike: deterministic, the same everywhere.
+// (GB300 adds two FP64 lanes a clock: the 32 warps' FP64 shuffle trees cost 3400
+// clocks a sum, the pairs some 600; and one thread divides, as 1024 FP64
+// divisions took 5000 clocks.)  A warp whose pair sum leaves the FP32 range adds
+// in FP64.
+template <int NV, typename F>
+__device__ __forceinline__ bool meet(Meeting& m, const float (&t)[NV], double* const (&part)[NV], int lb, int nb,
+                                     float& result, F finish) {
+  __shared__ float wsum[NV][2][kCgThreads / 32];
+  __shared__ double wide[NV][kCgThreads / 32];  // of warps whose pair sum left the FP32 range
+  __shared__ float answer;
   __shared__ int ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ok = 1;
-    const unsigned g = ld_acquire(&s->gen);
-    if (atom_add_acq_rel(&s->count, 1u) == gridDim.x - 1 && !bias) {
-      s->count = 0u;  // ordered before the release below; nobody arrives until it
-      atom_add_acq_rel(&s->gen, 1u);
-    } else {
-      const unsigned long long t0 = global_ns();
-      unsigned polls = 0;
-      while (ld_acquire(&s->gen) == g) {
-        if ((++polls & 255u) == 0 &&
-            ((long long)(global_ns() - t0) > limit_ns || (*(volatile int*)status & kStatusBarrier))) {
-          atomicOr(status, kStatusBarrier);
-          ok = 0;
-          break;
-        }
-      }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    float s = t[i], e = 0.f;
+#pragma unroll
+    for (int o = 16; o; o >>= 1)
+      pair_add(s, e, __shfl_xor_sync(0xffffffffu, s, o), __shfl_xor_sync(0xffffffffu, e, o));
+    if (lane == 0) {
+      wsum[i][0][warp] = s;
+      wsum[i][1][warp] = e;
+    }
+    if (!isfinite(s)) {  // (the same in all lanes)
+      const double d = warp_sum((double)t[i]);
+      if (lane == 0) wide[i][warp] = d;
     }
   }
   __syncthreads();
+  ++m.passed;
+  if (warp == 0) {
+    double mine[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const float s0 = wsum[i][0][lane], e0 = wsum[i][1][lane];
+      float s = s0, e = e0;
+#pragma unroll
+      for (int o = 16; o; o >>= 1)
+        pair_add(s, e, __shfl_xor_sync(0xffffffffu, s, o), __shfl_xor_sync(0xffffffffu, e, o));
+      mine[i] = isfinite(s) ? (double)s + (double)e
+                            : warp_sum(isfinite(s0) ? (double)s0 + (double)e0 : wide[i][lane]);
+    }
+    int fine = 1;
+    if (lane == 0) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) part[i][lb] = mine[i];
+      const unsigned target = m.passed * gridDim.x + m.bias;
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&m.sync->count) : "memory");
+      if ((int)(ld_relaxed(&m.sync->count) - target) < 0) {
+        const unsigned long long t0 = global_ns();
+        unsigned polls = 0;
+        while ((int)(ld_relaxed(&m.sync->count) - target) < 0) {
+          if ((++polls & 255u) == 0 &&
+              ((long long)(global_ns() - t0) > m.limit_ns || (*(volatile int*)m.status & kStatusBarrier))) {
+            atomicOr(m.status, kStatusBarrier);
+            fine = 0;
+            break;
+          }
+        }
+      }
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    }
+    __syncwarp();
+    double sums[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      constexpr int kAtOnce = 5;  // loads in flight: 160 blocks at a time
+      double u = 0.0;
+      for (int b0 = 0; b0 < nb; b0 += 32 * kAtOnce) {
+        double v[kAtOnce];
+#pragma unroll
+        for (int k = 0; k < kAtOnce; ++k) {
+          const int b = b0 + 32 * k + lane;
+          v[k] = b < nb ? *(volatile const double*)(part[i] + b) : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < kAtOnce; ++k) u += v[k];
+      }
+      sums[i] = warp_sum(u);
+    }
+    if (lane == 0) {
+      answer = finish(sums);
+      ok = fine;
+    }
+  }
+  __syncthreads();
+  result = answer;
   return ok != 0;
 }
 
@@ -285,15 +341,38 @@ __global__ void __launch_bounds__(kThreads) dsa_stencil_kernel(DsaGeom g, const 
   }
 }
 
-// assembled sigma_s0 M v_0 at vertex (I, J, K): for each cell around the
-// vertex, the cell's nodal values times the row of the mixed mass matrix
-// (vertex hat function x the cell's DG Q_p basis, cell measure folded in) of
-// the corner the vertex is for that cell
+// The residual's cell moments: for each cell its nodal values times the rows of the
+// mixed mass matrix (vertex hat functions x the cell's DG Q_p basis, cell measure
+// folded in), one value per corner.  A thread per cell, so each FP64 value is
+// converted once (two lanes a clock; the vertices used to convert the values of all
+// the cells around them, eight times each: 40 us on 64^3).
 template <int DIM>
-__device__ __forceinline__ float assemble_rhs(const DsaGeom& g, const float4* __restrict__ cell,
-                                              const double* __restrict__ v, int I, int J, int K,
-                                              const float* __restrict__ smix, int n) {
-  constexpr int NC = DIM == 3 ? 2 : 1;
+__device__ __forceinline__ void cell_moments(const DsaGeom& g, const double* __restrict__ v, const float* smix, int n,
+                                             float* __restrict__ cm, int first, int stride) {
+  constexpr int NCORNER = DIM == 3 ? 8 : 4;
+  const int nc = g.nx * g.ny * g.nz;
+  for (int c = first; c < nc; c += stride) {
+    const double* vc = v + (long)c * n;
+    float sm[NCORNER];
+#pragma unroll
+    for (int cr = 0; cr < NCORNER; ++cr) sm[cr] = 0.f;
+    for (int j = 0; j < n; ++j) {
+      const float vj = (float)vc[j];
+#pragma unroll
+      for (int cr = 0; cr < NCORNER; ++cr) sm[cr] += smix[cr * n + j] * vj;
+    }
+#pragma unroll
+    for (int cr = 0; cr < NCORNER; cr += 4)
+      reinterpret_cast<float4*>(cm + (long)c * NCORNER)[cr / 4] = make_float4(sm[cr], sm[cr + 1], sm[cr + 2], sm[cr + 3]);
+  }
+}
+
+// assembled sigma_s0 M v_0 at vertex (I, J, K): for each cell around the vertex the
+// moment of the corner the vertex is for that cell
+template <int DIM>
+__device__ __forceinline__ float assemble_rhs(const DsaGeom& g, const float4* __restrict__ cell, const float* cm, int I,
+                                              int J, int K) {
+  constexpr int NC = DIM == 3 ? 2 : 1, NCORNER = DIM == 3 ? 8 : 4;
   float acc = 0.f;
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
@@ -308,15 +387,51 @@ __device__ __forceinline__ float assemble_rhs(const DsaGeom& g, const float4* __
         const int kx = I - 1 + a;
         if (kx < 0 || kx >= g.nx) continue;
         const int cid = (kz * g.ny + ky) * g.nx + kx;
-        const double* vc = v + (long)cid * n;
-        const float* row = smix + ((1 - a) + 2 * (1 - b) + (DIM == 3 ? 4 * (1 - c) : 0)) * n;
-        float sm = 0.f;
-        for (int j = 0; j < n; ++j) sm += row[j] * (float)vc[j];
-        acc += __ldg(&cell[cid].z) * sm;
+        const int cr = (1 - a) + 2 * (1 - b) + (DIM == 3 ? 4 * (1 - c) : 0);
+        acc += __ldg(&cell[cid].z) * cm[(long)cid * NCORNER + cr];
       }
     }
   }
   return acc;
+}
+
+// out = v + f, the vertex field f (at(vertex)) interpolated from the cell's corner
+// vertices at each scalar-moment node (Q1: the node is the vertex)
+template <int DIM, typename F>
+__device__ __forceinline__ void write_out(const DsaGeom& g, const double* v, double* out, long len, long n0, int first,
+                                          int stride, int n, const float* sipl, F at) {
+  constexpr int NCORNER = DIM == 3 ? 8 : 4;
+  const bool small = n0 < (1L << 31);  // 32-bit index arithmetic
+  for (long e = first; e < len; e += stride) {
+    double val = v[e];
+    if (e < n0) {
+      int cid, k;
+      if (n == NCORNER) {
+        cid = (int)(e / NCORNER);
+        k = (int)(e % NCORNER);
+      } else if (small) {
+        cid = (int)((unsigned)e / (unsigned)n);
+        k = (int)((unsigned)e - (unsigned)cid * (unsigned)n);
+      } else {
+        cid = (int)(e / n);
+        k = (int)(e % n);
+      }
+      const int tt = cid / g.nx, kx = cid - tt * g.nx;
+      const int kz = DIM == 3 ? tt / g.ny : 0, ky = tt - kz * g.ny;
+      const int v0 = (kz * g.vy + ky) * g.vx + kx;  // the cell's corner (0, 0, 0)
+      float f = 0.f;
+      if (n == NCORNER) {
+        f = at(v0 + (DIM == 3 ? (k >> 2) * g.vy * g.vx : 0) + ((k >> 1) & 1) * g.vx + (k & 1));
+      } else {
+#pragma unroll
+        for (int cr = 0; cr < NCORNER; ++cr)
+          f += sipl[k * NCORNER + cr] *
+               at(v0 + (DIM == 3 ? (cr >> 2) * g.vy * g.vx : 0) + ((cr >> 1) & 1) * g.vx + (cr & 1));
+      }
+      val += (double)f;
+    }
+    out[e] = val;
+  }
 }
 
 // The whole preconditioner of one problem: assemble the right-hand side,
@@ -336,7 +451,7 @@ __device__ __forceinline__ void cg_body(const DsaGeom& g, const float4* __restri
                                         float* p, float* q, double* part_a, double* part_b, int lb, int nb,
                                         DsaSync* sync, int* status, long long limit_ns, int iters,
                                         const float* __restrict__ fe, int n, const float* __restrict__ x0,
-                                        double* part_c, unsigned wait_bias) {
+                                        double* part_c, unsigned wait_bias, float* cm) {
   constexpr int NCORNER = DIM == 3 ? 8 : 4;
   // the cell tables: mixed mass [corner][n] (measure folded in), then the
   // interpolation of the vertex values at the nodes [n][corner]
@@ -348,39 +463,40 @@ __device__ __forceinline__ void cg_body(const DsaGeom& g, const float4* __restri
   __syncthreads();
   const int stride = nb * kCgThreads;
   const int first = lb * kCgThreads + threadIdx.x;
+  Meeting m{sync, status, limit_ns, wait_bias};
+  float res = 0.f;
+  cell_moments<DIM>(g, v, smix, n, cm, first, stride);
+  {
+    const float none[1] = {0.f};
+    if (!meet<1>(m, none, {x0 ? part_b : part_a}, lb, nb, res, [](const double*) { return 0.f; })) return;
+  }
   // x = 0, r = rhs without a guess.  With a guess g (x0, written before the
   // launch with a zero halo like z, so every block reads its neighbours'
   // values without a barrier) the start is the multiple of g closest to the
   // solution in the energy norm, x = a g with a = (g, rhs) / (g, C g) (a
   // Galerkin step on span{g}: never farther from the solution than x = 0,
   // whatever the guess), and r = rhs - a C g (C g kept in q meanwhile).
-  float t = 0.f;
   float a0 = 0.f;
   if (x0) {
-    float t1 = 0.f, t2 = 0.f;
+    float t[2] = {0.f, 0.f};
     for (int vid = first; vid < g.nv; vid += stride) {
       int I, J, K;
       vertex_ijk(g, vid, I, J, K);
-      const float rr = assemble_rhs<DIM>(g, cell, v, I, J, K, smix, n);
+      const float rr = assemble_rhs<DIM>(g, cell, cm, I, J, K);
       float w = 0.f;
 #pragma unroll
       for (int s = 0; s < kStencil<DIM>; ++s) w += coef[(long)s * g.nv + vid] * x0[vid + g.off[s]];
       r[vid] = rr;
       q[vid] = w;
-      t1 += x0[vid] * rr;
-      t2 += x0[vid] * w;
+      t[0] += x0[vid] * rr;
+      t[1] += x0[vid] * w;
     }
-    // part_c is written here only, so no later phase overwrites it while a
-    // slower block still reads it; part_a is next written after a barrier
-    const double b1 = block_sum(t1), b2 = block_sum(t2);
-    if (threadIdx.x == 0) {
-      part_a[lb] = b1;
-      part_c[lb] = b2;
-    }
-    if (!grid_barrier(sync, status, limit_ns, wait_bias)) return;
-    const double gb = all_sum(part_a, nb), gcg = all_sum(part_c, nb);
-    a0 = gcg > 0.0 ? (float)(gb / gcg) : 0.f;
+    if (!meet<2>(m, t, {part_a, part_c}, lb, nb, a0,
+                 [](const double* u) { return u[1] > 0.0 ? (float)(u[0] / u[1]) : 0.f; }))
+      return;
   }
+  double rz = 0.0;  // (thread 0's)
+  float t[1] = {0.f};
   for (int vid = first; vid < g.nv; vid += stride) {
     float rr, xx = 0.f;
     if (x0) {
@@ -389,22 +505,23 @@ __device__ __forceinline__ void cg_body(const DsaGeom& g, const float4* __restri
     } else {
       int I, J, K;
       vertex_ijk(g, vid, I, J, K);
-      rr = assemble_rhs<DIM>(g, cell, v, I, J, K, smix, n);
+      rr = assemble_rhs<DIM>(g, cell, cm, I, J, K);
     }
     const float zz = rr * dinv[vid];
     r[vid] = rr;
     z[vid] = zz;
     x[vid] = xx;
-    t += rr * zz;
+    t[0] += rr * zz;
   }
-  double bt = block_sum(t);
-  if (threadIdx.x == 0) part_b[lb] = bt;
-  if (!grid_barrier(sync, status, limit_ns, wait_bias)) return;
-  double rz = all_sum(part_b, nb), beta = 0.0, alpha = 0.0;
+  if (!meet<1>(m, t, {part_b}, lb, nb, res, [&](const double* u) {
+        rz = u[0];
+        return 0.f;
+      }))
+    return;
+  float fa = 0.f, fb = 0.f;
   for (int it = 0; it < iters; ++it) {
     // w = C z; p = z + beta p; q = w + beta q
-    const float fb = (float)beta;
-    t = 0.f;
+    t[0] = 0.f;
     for (int vid = first; vid < g.nv; vid += stride) {
       // z has a zero halo: every stencil offset stays inside the buffer, and
       // entries that wrap to another row have coefficient 0
@@ -416,60 +533,31 @@ __device__ __forceinline__ void cg_body(const DsaGeom& g, const float4* __restri
       const float qn = it ? w + fb * q[vid] : w;
       p[vid] = pn;
       q[vid] = qn;
-      t += pn * qn;
+      t[0] += pn * qn;
     }
-    bt = block_sum(t);
-    if (threadIdx.x == 0) part_a[lb] = bt;
-    if (!grid_barrier(sync, status, limit_ns, wait_bias)) return;
-    const double pq = all_sum(part_a, nb);
-    alpha = pq > 0.0 ? rz / pq : 0.0;
+    if (!meet<1>(m, t, {part_a}, lb, nb, fa,
+                 [&](const double* u) { return u[0] > 0.0 ? (float)(rz / u[0]) : 0.f; }))
+      return;
     if (it == iters - 1) break;  // the last update folds into the output
     // x += alpha p; r -= alpha q; z = r / diag
-    const float fa = (float)alpha;
-    t = 0.f;
+    t[0] = 0.f;
     for (int vid = first; vid < g.nv; vid += stride) {
       x[vid] += fa * p[vid];
       const float rn = r[vid] - fa * q[vid];
       const float zn = rn * dinv[vid];
       r[vid] = rn;
       z[vid] = zn;
-      t += rn * zn;
+      t[0] += rn * zn;
     }
-    bt = block_sum(t);
-    if (threadIdx.x == 0) part_b[lb] = bt;
-    if (!grid_barrier(sync, status, limit_ns, wait_bias)) return;
-    const double rzn = all_sum(part_b, nb);
-    beta = rz > 0.0 ? rzn / rz : 0.0;
-    rz = rzn;
+    if (!meet<1>(m, t, {part_b}, lb, nb, fb, [&](const double* u) {
+          const float beta = rz > 0.0 ? (float)(u[0] / rz) : 0.f;
+          rz = u[0];
+          return beta;
+        }))
+      return;
   }
-  // out = v + f, f = x + alpha p interpolated from the cell's corner vertices
-  // at each scalar-moment node (Q1: the node is the vertex); x and p of other
-  // blocks' vertices are complete at the last barrier
-  const float fa = (float)alpha;
-  for (long e = first; e < len; e += stride) {
-    double val = v[e];
-    if (e < n0) {
-      const long cid = e / n;
-      const int k = (int)(e % n);
-      const int kx = (int)(cid % g.nx);
-      const long tt = cid / g.nx;
-      const int ky = (int)(tt % g.ny), kz = (int)(tt / g.ny);
-      const long v0 = ((long)kz * g.vy + ky) * g.vx + kx;  // the cell's corner (0, 0, 0)
-      float f = 0.f;
-      if (n == NCORNER) {
-        const long vid = v0 + (DIM == 3 ? (long)(k >> 2) * g.vy * g.vx : 0) + ((k >> 1) & 1) * g.vx + (k & 1);
-        f = x[vid] + fa * p[vid];
-      } else {
-#pragma unroll
-        for (int cr = 0; cr < NCORNER; ++cr) {
-          const long vid = v0 + (DIM == 3 ? (long)(cr >> 2) * g.vy * g.vx : 0) + ((cr >> 1) & 1) * g.vx + (cr & 1);
-          f += sipl[k * NCORNER + cr] * (x[vid] + fa * p[vid]);
-        }
-      }
-      val += (double)f;
-    }
-    out[e] = val;
-  }
+  // x and p of other blocks' vertices are complete at the last meeting
+  write_out<DIM>(g, v, out, len, n0, first, stride, n, sipl, [&](int i) { return x[i] + fa * p[i]; });
 }
 
 template <int DIM>
@@ -482,9 +570,153 @@ __global__ void __launch_bounds__(kCgThreads, 1) dsa_cg_kernel(DsaGeom g, const 
                                                           long long limit_ns, int iters,
                                                           const float* __restrict__ fe, int n,
                                                           const float* __restrict__ x0, double* part_c,
-                                                          unsigned wait_bias) {
+                                                          unsigned wait_bias, float* cm) {
   cg_body<DIM>(g, cell, coef, v, out, len, n0, dinv, x, r, z, p, q, part_a, part_b, (int)blockIdx.x,
-               (int)gridDim.x, sync, status, limit_ns, iters, fe, n, x0, part_c, wait_bias);
+               (int)gridDim.x, sync, status, limit_ns, iters, fe, n, x0, part_c, wait_bias, cm);
+}
+
+// The same solve with everything but z on chip: a thread keeps its KV vertices' x,
+// r, p, q and 1/diag in registers and their stencil rows in shared memory (64^3:
+// 1807 vertices x 27 x 4 B = 195 KB a block), so a CG step reads z of the neighbours
+// and nothing else through L2.  With the tables streamed from L2 and the vectors in
+// global memory a step of the 64^3 mesh moved 29.7 MB of coefficients and some 10 MB of
+// vectors; 20 steps took 484 us there, before the sums of meet(), and 213 us here: two
+// meetings a step of some 3 us, the matrix row 1.8, the update and its vectors the rest.
+// Blocks own runs of KV x 1024 vertices, so most neighbours are the block's own.
+template <int DIM, int KV>
+__global__ void __launch_bounds__(kCgThreads, 1)
+    dsa_cg_resident_kernel(DsaGeom g, const float4* __restrict__ cell, const float* __restrict__ coef, const double* v,
+                           double* out, long len, long n0, const float* __restrict__ dinv, float* xg, float* pg, float* z,
+                           double* part_a, double* part_b, DsaSync* sync, int* status, long long limit_ns, int iters,
+                           const float* __restrict__ fe, int n, const float* __restrict__ x0, double* part_c,
+                           unsigned wait_bias, float* cm) {
+  constexpr int NCORNER = DIM == 3 ? 8 : 4, NS = kStencil<DIM>;
+  extern __shared__ float scoef[];  // [KV][NS][kCgThreads]
+  __shared__ float smix[NCORNER * kMaxNodes], sipl[kMaxNodes * NCORNER];
+  const int tid = threadIdx.x, lb = (int)blockIdx.x, nb = (int)gridDim.x;
+  // the stencil rows are on their way while the right-hand side is formed (a
+  // thread copies and reads its own)
+  int vid[KV];
+#pragma unroll
+  for (int k = 0; k < KV; ++k) {
+    vid[k] = (lb * KV + k) * kCgThreads + tid;
+    if (vid[k] < g.nv) {
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        const unsigned to = (unsigned)__cvta_generic_to_shared(scoef + (k * NS + s) * kCgThreads + tid);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(coef + (long)s * g.nv + vid[k])
+                     : "memory");
+      }
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int k = tid; k < NCORNER * n; k += kCgThreads) {
+    smix[k] = fe[k];
+    sipl[k] = fe[NCORNER * n + k];
+  }
+  float x[KV], r[KV], p[KV], q[KV], di[KV];
+#pragma unroll
+  for (int k = 0; k < KV; ++k) {
+    x[k] = r[k] = p[k] = q[k] = 0.f;
+    di[k] = vid[k] < g.nv ? dinv[vid[k]] : 0.f;
+  }
+  __syncthreads();  // smix, sipl
+  Meeting m{sync, status, limit_ns, wait_bias};
+  float res = 0.f;
+  cell_moments<DIM>(g, v, smix, n, cm, lb * kCgThreads + tid, nb * kCgThreads);
+  {
+    const float none[1] = {0.f};
+    const bool ok = meet<1>(m, none, {x0 ? part_b : part_a}, lb, nb, res, [](const double*) { return 0.f; });
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (!ok) return;
+  }
+  auto row = [&](const float* f, int k) {  // the matrix row of vertex k applied to f
+    float w = 0.f;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) w += scoef[(k * NS + s) * kCgThreads + tid] * f[vid[k] + g.off[s]];
+    return w;
+  };
+  {
+    float t[2] = {0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < KV; ++k)
+      if (vid[k] < g.nv) {
+        int I, J, K;
+        vertex_ijk(g, vid[k], I, J, K);
+        r[k] = assemble_rhs<DIM>(g, cell, cm, I, J, K);
+        if (x0) {  // the guess's energy-optimal multiple (cg_body); C x0 kept in q
+          q[k] = row(x0, k);
+          x[k] = x0[vid[k]];
+          t[0] += x[k] * r[k];
+          t[1] += x[k] * q[k];
+        }
+      }
+    if (x0) {
+      float a0 = 0.f;
+      if (!meet<2>(m, t, {part_a, part_c}, lb, nb, a0,
+                   [](const double* u) { return u[1] > 0.0 ? (float)(u[0] / u[1]) : 0.f; }))
+        return;
+#pragma unroll
+      for (int k = 0; k < KV; ++k) {
+        r[k] -= a0 * q[k];
+        x[k] *= a0;
+      }
+    }
+  }
+  double rz = 0.0;  // (thread 0's)
+  float t[1] = {0.f};
+#pragma unroll
+  for (int k = 0; k < KV; ++k)
+    if (vid[k] < g.nv) {
+      const float zz = r[k] * di[k];
+      z[vid[k]] = zz;
+      t[0] += r[k] * zz;
+    }
+  if (!meet<1>(m, t, {part_b}, lb, nb, res, [&](const double* u) {
+        rz = u[0];
+        return 0.f;
+      }))
+    return;
+  float fa = 0.f, fb = 0.f;
+  for (int it = 0; it < iters; ++it) {
+    t[0] = 0.f;
+#pragma unroll
+    for (int k = 0; k < KV; ++k)
+      if (vid[k] < g.nv) {
+        const float w = row(z, k);
+        const float zz = r[k] * di[k];  // z of the thread's own vertex
+        p[k] = it ? zz + fb * p[k] : zz;
+        q[k] = it ? w + fb * q[k] : w;
+        t[0] += p[k] * q[k];
+        if (it == iters - 1) {  // the output reads every vertex's x + alpha p
+          xg[vid[k]] = x[k];
+          pg[vid[k]] = p[k];
+        }
+      }
+    if (!meet<1>(m, t, {part_a}, lb, nb, fa,
+                 [&](const double* u) { return u[0] > 0.0 ? (float)(rz / u[0]) : 0.f; }))
+      return;
+    if (it == iters - 1) break;
+    t[0] = 0.f;
+#pragma unroll
+    for (int k = 0; k < KV; ++k) {
+      x[k] += fa * p[k];
+      r[k] -= fa * q[k];
+      if (vid[k] < g.nv) {
+        const float zn = r[k] * di[k];
+        z[vid[k]] = zn;
+        t[0] += r[k] * zn;
+      }
+    }
+    if (!meet<1>(m, t, {part_b}, lb, nb, fb, [&](const double* u) {
+          const float beta = rz > 0.0 ? (float)(u[0] / rz) : 0.f;
+          rz = u[0];
+          return beta;
+        }))
+      return;
+  }
+  write_out<DIM>(g, v, out, len, n0, lb * kCgThreads + tid, nb * kCgThreads, n, sipl, 
+                 [&](int i) { return xg[i] + fa * pg[i]; });
 }
 
 // One problem of a batched diffusion solve: its tables, vectors and the
@@ -494,7 +726,7 @@ struct DsaProb {
   const float4* cell;
   const float* coef;
   const float* dinv;
-  float *x, *r, *z, *p, *q;
+  float *x, *r, *z, *p, *q, *cm;
   const float* fe;
   const double* v;
   double* out;
@@ -517,7 +749,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) dsa_cg_batch_kernel(const DsaPr
   const int lb = (int)blockIdx.x - P.block0;
   cg_body<DIM>(P.g, P.cell, P.coef, P.v, P.out, P.len, P.n0, P.dinv, P.x, P.r, P.z, P.p, P.q,
                part_a + P.block0, part_b + P.block0, lb, P.nblk, sync, status, limit_ns, iters, P.fe, P.n,
-               nullptr, nullptr, 0u);
+               nullptr, nullptr, 0u, P.cm);
 }
 
 int dfail(ouranos_rt* rt, cudaError_t e, const char* what) {
@@ -662,6 +894,7 @@ int ensure_tables(ouranos_rt* rt) {
   // x, r, p, q, 1/diag, z and the initial guess x0, the last two with zero halos
   DC(rt->d_dsa_vec.alloc(sizeof(float) * (7 * nv + 4 * halo(g))), "vectors");
   DC(rt->d_dsa_coef.alloc(sizeof(float) * ns * nv), "stencil");
+  DC(rt->d_dsa_cm.alloc(sizeof(float) * (rt->dim == 3 ? 8 : 4) * rt->n_cells), "cell moments");
   DC(cudaMemsetAsync(rt->d_dsa_vec.p, 0, sizeof(float) * (7 * nv + 4 * halo(g)), rt->stream), "vectors");
   // partials of the two phases (one per block of the cooperative grid) and the barrier
   int per_sm = 0, sms = 0;
@@ -724,8 +957,30 @@ int dsa_run(ouranos_rt* rt, const double* v, double* out, int iters, bool guess)
   const float* fe = rt->d_dsa_fe.as<float>();
   int n = rt->n;
   unsigned bias = rt->wait_bias ? 1u : 0u;  // the test hook of ouranos_rt_debug_wait_bias
+  float* cm = rt->d_dsa_cm.as<float>();
+  // on chip where the block's stencil rows fit its shared memory
+  const long per_thread = (nv + (long)rt->dsa_grid * kCgThreads - 1) / ((long)rt->dsa_grid * kCgThreads);
+  const int kv = (int)per_thread;
+  if (kv <= (DIM == 3 ? 2 : 6)) {
+    void* rargs[] = {&g, &cell, &coef, &v, &out, &len, &n0, &dinv, &x, &p, &z, &part_a, &part_b, &sync, &status,
+                     &limit, &iters, &fe, &n, &x0, &part_c, &bias, &cm};
+    const void* k1 = (const void*)dsa_cg_resident_kernel<DIM, 1>;
+    const void* k2 = (const void*)dsa_cg_resident_kernel<DIM, 2>;
+    const void* fn = kv == 1 ? k1 : k2;
+    int held = kv <= 2 ? kv : 2;
+    if constexpr (DIM == 2) {
+      if (kv > 2) {
+        held = kv <= 4 ? 4 : 6;
+        fn = kv <= 4 ? (const void*)dsa_cg_resident_kernel<2, 4> : (const void*)dsa_cg_resident_kernel<2, 6>;
+      }
+    }
+    const size_t smem = sizeof(float) * held * kStencil<DIM> * kCgThreads;
+    DC(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "solve");
+    DC(cudaLaunchCooperativeKernel(fn, dim3(rt->dsa_grid), dim3(kCgThreads), rargs, smem, rt->stream), "solve");
+    return OURANOS_OK;
+  }
   void* args[] = {&g, &cell, &coef, &v, &out, &len, &n0, &dinv, &x, &r, &z, &p, &q, &part_a, &part_b, &sync, &status,
-                  &limit, &iters, &fe, &n, &x0, &part_c, &bias};
+                  &limit, &iters, &fe, &n, &x0, &part_c, &bias, &cm};
   DC(cudaLaunchCooperativeKernel((const void*)dsa_cg_kernel<DIM>, dim3(rt->dsa_grid), dim3(kCgThreads), args, 0,
                                  rt->stream),
      "solve");
@@ -790,6 +1045,7 @@ int dsa_batch_launch(ouranos_rt* const* rts, const double* const* v, double* con
     P.q = base + 3 * n;
     P.dinv = base + 4 * n;
     P.z = base + 5 * n + halo(P.g);
+    P.cm = rt->d_dsa_cm.as<float>();
     P.cell = rt->d_dsa_cell.as<float4>();
     P.coef = rt->d_dsa_coef.as<float>();
     P.fe = rt->d_dsa_fe.as<float>();
