@@ -432,10 +432,12 @@ int setup_group(ouranos_rt* rt) {
     const long NS = rt->nx[rt->dim - 1], ncol = rt->n_cells / NS, words = (NS + 3) / 4;
     std::vector<unsigned> packed((size_t)2 * words * ncol, 0u);
     for (int dir = 0; dir < 2; ++dir)
-      for (long k = 0; k < NS; ++k)
-        for (long c = 0; c < ncol; ++c)
-          packed[((size_t)dir * words + k / 4) * ncol + c] |=
-              (unsigned)ccls[c + ncol * (dir ? NS - 1 - k : k)] << (8 * (k % 4));
+      for (long k = 0; k < NS; ++k) {
+        unsigned* to = &packed[((size_t)dir * words + k / 4) * ncol];
+        const int* from = &ccls[ncol * (dir ? NS - 1 - k : k)];
+        const int shift = 8 * (int)(k % 4);
+        for (long c = 0; c < ncol; ++c) to[c] |= (unsigned)from[c] << shift;
+      }
     OK_OR_RETURN(upload(rt, rt->d_cls4, packed, "cell classes"));
   }
   // A'^-1 per (sigma class, |Omega| class)

@@ -13,6 +13,11 @@
 //     bytes) into a shared ring, and psi and the edge words leave through a
 //     shared slot the same way; a lane copying its own cell met 32 lines per
 //     instruction, one clock each;
+//   - in FP32 the 32 bytes of a 3-D Q1 cell leave their lane in one store, 32 clocks
+//     of that pipe (through the slot 56: two-way conflicts going in, the read, two
+//     stores of 16 lines), and its source is read 16 bytes at a time: sweep kernel of
+//     128^3 LS S8 4604 -> 4100 us.  In 2-D the cells of 32 (FP64) and 16 bytes
+//     measured the same within 4 % either way and take the slot;
 //   - the face mass matrices are kernel arguments (constant memory);
 //   - a column's materials come four planes to a word.
 // Every dof is rounded in the order of the other forms, so all give the same bits.
@@ -37,7 +42,10 @@ struct LaneSlot {
   static constexpr int PF = 2, RING = PF + 1;             // planes in flight ahead of the one being solved
   static constexpr int WX = DIM == 2 ? 32 : 4, WY = 32 / WX;
   static constexpr int EB = (FD * SZ + 15) / 16 * 16;     // an edge's face values
-  static constexpr int o_ex = 32 * OUT;
+  // one store per cell: the slot holds the outflow edges only
+  static constexpr bool kDirect = DIM == 3 && P1 == 2 && SZ == 4;
+  static constexpr int o_ox = 0, o_oy = WY * EB;
+  static constexpr int o_ex = kDirect ? (WY + WX) * EB : 32 * OUT;
   static constexpr int o_ey = o_ex + WY * EB;
   static constexpr int o_cls = o_ey + (DIM == 3 ? WX * EB : 0);
   static constexpr int CW = 4;                            // class words in flight per column
@@ -52,6 +60,46 @@ __device__ __forceinline__ uint4 ldg_first(const unsigned char* p) {
                : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w)
                : "l"(p));
   return u;
+}
+
+// FD values of an edge slot: 16 bytes a load, or one value where registers are short
+template <bool VEC, int FD, typename real, int NV>
+__device__ __forceinline__ void load_edge(real (&v)[NV], const unsigned char* from) {
+  if constexpr (VEC) {
+#pragma unroll
+    for (int k = 0; k < NV * (int)sizeof(real) / 16; ++k) {
+      const uint4 u = *reinterpret_cast<const uint4*>(from + 16 * k);
+      memcpy(v + k * (16 / sizeof(real)), &u, 16);
+    }
+  } else {
+#pragma unroll
+    for (int t = 0; t < FD; ++t) v[t] = *reinterpret_cast<const real*>(from + t * sizeof(real));
+  }
+}
+
+// the pairs of a Q1 cell between canonical and physical order: pair m of the one is
+// pair m ^ flips of the other, its values swapped where x is flipped
+__device__ __forceinline__ void flip_pairs(f2 (&v)[4], int flip) {
+#pragma unroll
+  for (int m = 0; m < 4; ++m) v[m] = Pk<float>::swap_if(v[m], flip & 1);
+#pragma unroll
+  for (int ax = 1; ax < 3; ++ax) {
+    const bool f = flip & (1 << ax);
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+      if (!(m & ax)) {
+        const f2 lo = v[m], hi = v[m | ax];
+        v[m] = f ? hi : lo;
+        v[m | ax] = f ? lo : hi;
+      }
+  }
+}
+// eight FP32 values in one streaming store of 32 bytes
+__device__ __forceinline__ void store_cell(void* to, const f2 (&v)[4]) {
+  asm volatile("st.global.cs.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(to), "f"(f2_get(v[0], 0)),
+               "f"(f2_get(v[0], 1)), "f"(f2_get(v[1], 0)), "f"(f2_get(v[1], 1)), "f"(f2_get(v[2], 0)),
+               "f"(f2_get(v[2], 1)), "f"(f2_get(v[3], 0)), "f"(f2_get(v[3], 1))
+               : "memory");
 }
 
 template <typename real, int DIM, int P1, int FM>
@@ -281,16 +329,16 @@ __device__ __forceinline__ void sweep_lane_task(const SweepArgs<real>& a, const 
     cp_async_wait<S::PF - 1>();  // this step's sources have landed
     __syncwarp();
     // ---- upwind face values: the neighbour's outflow, or the edge slot's
-    real upX[FD], upY[DIM == 3 ? FD : 1];
+    real upX[FD], upY[DIM == 3 ? FD : 1], ex[S::EB / SZ], ey[S::EB / SZ];
+    load_edge<S::kDirect, FD>(ex, sm + S::o_ex + ly * S::EB);
+    if (DIM == 3) load_edge<S::kDirect, FD>(ey, sm + S::o_ey + lx * S::EB);
 #pragma unroll
     for (int t = 0; t < FD; ++t) {
       const real sx = A::shfl_up(psiX[t], 1);
-      const real ex = *reinterpret_cast<const real*>(sm + S::o_ex + ly * S::EB + t * SZ);
-      upX[t] = lx == 0 ? ex : sx;
+      upX[t] = lx == 0 ? ex[t] : sx;
       if constexpr (DIM == 3) {
         const real sy = A::shfl_up(psiY[t], WX);
-        const real ey = *reinterpret_cast<const real*>(sm + S::o_ey + lx * S::EB + t * SZ);
-        upY[t] = ly == 0 ? ey : sy;
+        upY[t] = ly == 0 ? ey[t] : sy;
       }
     }
     // ---- material of this plane (class 0 for idle lanes)
@@ -304,7 +352,10 @@ __device__ __forceinline__ void sweep_lane_task(const SweepArgs<real>& a, const 
     // the first columns of the inverse, on their way while b is formed
     constexpr int PJ = 8 / SZ, PL = 16 / SZ;  // columns per piece of a row pair, of the lone row
     constexpr int NCP = RW::pair_pieces(SZ);
-    constexpr int AHEAD = SZ == 8 ? 2 : 0;  // pieces of each row pair in flight
+    // pieces of each row pair in flight (Apply, us, with 0 / 1 / 2 / 3: 3-D Q1 64^3
+    // GLC S12 3993 / 3697 / 3908 / 4157, where registers are short; 2-D Q1 32^2
+    // 105 / 102 / 100 / -; FP32 3-D Q1 128^3 5382 / 5471 / 5552)
+    constexpr int AHEAD = SZ == 4 ? 0 : N == 8 ? 1 : 2;
     uint4 ring[AHEAD ? AHEAD : 1][RP];
 #pragma unroll
     for (int c = 0; c < AHEAD; ++c)
@@ -321,7 +372,33 @@ __device__ __forceinline__ void sweep_lane_task(const SweepArgs<real>& a, const 
         o0 = (int)((reinterpret_cast<size_t>(src0) + cb) & 15);
         if (FM >= 1) o1 = (int)((reinterpret_cast<size_t>(a.iso) + cb) & 15);
       }
-      if constexpr (P1 == 2) {
+      if constexpr (S::kDirect) {  // 16 bytes at a time: pairs at a stride of 48 bytes met two-way conflicts
+        P v[N / 2];
+        auto fetch_cell = [&](const unsigned char* from) {
+#pragma unroll
+          for (int c = 0; c < N / 4; ++c) {
+            const uint4 u = *reinterpret_cast<const uint4*>(from + 16 * c);
+            K::from16(u, v + 2 * c);
+          }
+          flip_pairs(v, flip);
+        };
+        typename K::Acc acc[N / 2];
+        if (FM >= 1) {
+          if (arrays == 2) fetch_cell(isrc);
+#pragma unroll
+          for (int m = 0; m < N / 2; ++m) acc[m] = K::from(arrays == 2 ? v[m] : K::make(real(0), real(0)));
+        }
+        fetch_cell(src);
+#pragma unroll
+        for (int m = 0; m < N / 2; ++m) {
+          if (FM >= 1) {
+            K::fma(acc[m], K::make(w0, w0), K::op(v[m]), z);
+            v[m] = K::raw(acc[m]);
+          }
+          b[2 * m] = K::get(v[m], 0);
+          b[2 * m + 1] = K::get(v[m], 1);
+        }
+      } else if constexpr (P1 == 2) {
 #pragma unroll
         for (int m = 0; m < N / 2; ++m) {
           const int at = (phys(2 * m) - (swap ? 1 : 0)) * SZ;
@@ -465,8 +542,14 @@ __device__ __forceinline__ void sweep_lane_task(const SweepArgs<real>& a, const 
         if (DIM == 3) psiY[DIM == 3 ? t : 0] = x[C::y_out(t)];
       }
     }
-    // ---- the cells' values, in physical order, into the shared slot
-    {
+    // ---- the cells' values, in physical order: to memory, the tile's outflow to its
+    // slot; or all into the shared slot
+    if constexpr (S::kDirect) {
+      if (px && lx == WX - 1)
+        for (int t = 0; t < FD; ++t) *reinterpret_cast<real*>(sm + S::o_ox + ly * S::EB + t * SZ) = x[C::x_out(t)];
+      if (DIM == 3 && py && ly == WY - 1)
+        for (int t = 0; t < FD; ++t) *reinterpret_cast<real*>(sm + S::o_oy + lx * S::EB + t * SZ) = x[C::y_out(t)];
+    } else {
       unsigned char* out = sm + lane * S::OUT;
       if constexpr (P1 == 2) {
 #pragma unroll
@@ -485,7 +568,7 @@ __device__ __forceinline__ void sweep_lane_task(const SweepArgs<real>& a, const 
         const int u = lane + 32 * k, e = edge_cell(k), r = s - (WX - 1) - e, g = e * WX + WX - 1;
         if (e < WY && ((on >> (g & 31)) & 1u)) {
           const int w = u - e * FW, i = phys(C::x_out(w / W)) * W + w % W;
-          const unsigned v = *reinterpret_cast<const unsigned*>(sm + g * S::OUT + i * 4);
+          const unsigned v = *reinterpret_cast<const unsigned*>(sm + (S::kDirect ? S::o_ox + e * S::EB + w * 4 : g * S::OUT + i * 4));
           st_relaxed_u64(out_x + (long)r * WY * FW + u, ((unsigned long long)((a.epoch << 16) | (unsigned)r) << 32) | v);
         }
       }
@@ -496,13 +579,20 @@ __device__ __forceinline__ void sweep_lane_task(const SweepArgs<real>& a, const 
         const int u = lane + 32 * k, e = edge_cell(k), r = s - (WY - 1) - e, g = (WY - 1) * WX + e;
         if (e < WX && ((on >> (g & 31)) & 1u)) {
           const int w = u - e * FW, i = phys(C::y_out(w / W)) * W + w % W;
-          const unsigned v = *reinterpret_cast<const unsigned*>(sm + g * S::OUT + i * 4);
+          const unsigned v = *reinterpret_cast<const unsigned*>(sm + (S::kDirect ? S::o_oy + e * S::EB + w * 4 : g * S::OUT + i * 4));
           st_relaxed_u64(out_y + (long)r * WX * FW + u, ((unsigned long long)((a.epoch << 16) | (unsigned)r) << 32) | v);
         }
       }
     }
     const int adv = s * cstep;
-    if constexpr (kAligned) {  // (the pieces are the source copies')
+    if constexpr (S::kDirect) {
+      P v[N / 2];
+#pragma unroll
+      for (int m = 0; m < N / 2; ++m) v[m] = K::make(x[2 * m], x[2 * m + 1]);
+      flip_pairs(v, flip);
+      if (act)
+        store_cell(reinterpret_cast<unsigned char*>(a.psi + dirbase) + (long)(col + cell0 + (s - skew) * cstep) * S::CELLB, v);
+    } else if constexpr (kAligned) {  // (the pieces are the source copies')
       unsigned char* pout = reinterpret_cast<unsigned char*>(a.psi + dirbase);
       auto piece = [&](int j) {
         const int u = lane + 32 * j, g = u / CH, p = u - g * CH;
@@ -538,7 +628,9 @@ __device__ __forceinline__ void sweep_lane_task(const SweepArgs<real>& a, const 
 template <typename real, int DIM, int P1>
 constexpr int lane_blocks() {
   constexpr int N = Cell<DIM, P1>::N;
-  return sizeof(real) == 8 ? (N == 4 ? 4 : N == 8 ? 3 : 2) : (N == 4 ? 6 : 4);
+  // (3-D Q1, Apply, us: FP32 128^3 with 3 / 4 / 5 / 6 blocks 6057 / 5382 / 5229 / 5913,
+  // FP64 64^3 with 3 / 4 blocks 3697 / 4707)
+  return sizeof(real) == 8 ? (N == 4 ? 4 : N == 8 ? 3 : 2) : (N == 4 ? 6 : N == 8 ? 5 : 4);
 }
 template <typename real, int DIM, int P1, int FM>
 __global__ void __launch_bounds__(128, (lane_blocks<real, DIM, P1>())) sweep_lane_kernel(const __grid_constant__ SweepArgs<real> a) {
