@@ -19,11 +19,48 @@ struct __align__(8) df64 {
   __host__ __device__ constexpr df64(float h, float l = 0.f) : hi(h), lo(l) {}
 };
 
+// Conversions on the integer pipe.  GB300's FP64 pipe takes two lanes a clock and
+// SM, conversions included: a split is four of its operations (two roundings, the
+// widening, the difference), 8 clocks a value, and the streaming kernels that split
+// their input were bound by it.  The same results from the bits: the significand's
+// 24 leading bits rounded to nearest even, and the rest, an integer of at most 29
+// bits, rounded by its own conversion.  Values outside the exponents where both
+// parts are normal (and infinities, NaN) take the FP64 pipe.
+
+// (float)x
+__device__ __forceinline__ float f32_from_f64(double x) {
+  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+  const unsigned e = (h >> 20) & 0x7ffu;
+  if (e - 897u <= 252u) {
+    const unsigned m = ((h & 0xfffffu) << 3) | (l >> 29), rest = l & 0x1fffffffu;
+    const unsigned up = rest > 0x10000000u || (rest == 0x10000000u && (m & 1u));
+    return __uint_as_float((h & 0x80000000u) | (((e - 896u) << 23) + m + up));
+  }
+  return ((h << 1) | l) == 0u ? __uint_as_float(h) : __double2float_rn(x);
+}
+// (double)f
+__device__ __forceinline__ double f64_from_f32(float f) {
+  const unsigned b = __float_as_uint(f), mag = b & 0x7fffffffu;
+  if ((mag >= 0x800000u && mag < 0x7f800000u) || mag == 0u)
+    return __hiloint2double((int)((b & 0x80000000u) | (mag ? (mag >> 3) + 0x38000000u : 0u)), (int)(b << 29));
+  return (double)f;
+}
+// hi = (float)x, lo = (float)(x - hi)
 __device__ __forceinline__ df64 df64_from(double x) {
+  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+  const unsigned e = (h >> 20) & 0x7ffu;
+  if (e - 949u <= 200u) {
+    const unsigned m = ((h & 0xfffffu) << 3) | (l >> 29), rest = l & 0x1fffffffu;
+    const unsigned up = rest > 0x10000000u || (rest == 0x10000000u && (m & 1u));
+    const int r = (int)rest - (int)(up << 29);  // x - hi in units of the last place
+    const float lo = (float)((int)h < 0 ? -r : r) * __uint_as_float((e - 948u) << 23);
+    return {__uint_as_float((h & 0x80000000u) | (((e - 896u) << 23) + m + up)), lo};
+  }
+  if (((h << 1) | l) == 0u) return {__uint_as_float(h), 0.f};
   const float hi = __double2float_rn(x);
   return {hi, __double2float_rn(x - (double)hi)};
 }
-__device__ __forceinline__ double df64_to(df64 a) { return (double)a.hi + (double)a.lo; }
+__device__ __forceinline__ double df64_to(df64 a) { return f64_from_f32(a.hi) + f64_from_f32(a.lo); }
 // the same split on the host (tables)
 inline df64 df64_split(double x) {
   const float hi = (float)x;
@@ -34,13 +71,15 @@ inline df64 df64_split(double x) {
 template <typename T>
 __device__ __forceinline__ T real_from_double(double x) { return (T)x; }
 template <>
+__device__ __forceinline__ float real_from_double<float>(double x) { return f32_from_f64(x); }
+template <>
 __device__ __forceinline__ df64 real_from_double<df64>(double x) { return df64_from(x); }
 template <typename T>
 __device__ __forceinline__ double real_to_double(T x) { return (double)x; }
 template <>
 __device__ __forceinline__ double real_to_double<df64>(df64 x) { return df64_to(x); }
 template <typename T>
-__device__ __forceinline__ df64 to_df64(T x) { return df64_from((double)x); }
+__device__ __forceinline__ df64 to_df64(T x) { return df64_from((double)x); }  // (T = double)
 template <>
 __device__ __forceinline__ df64 to_df64<df64>(df64 x) { return x; }
 

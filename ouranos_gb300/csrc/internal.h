@@ -279,7 +279,8 @@ cudaError_t launch_reduce_tc(const float* psi, const TcTables& t, float* phi, lo
 // phi[m][e] = sum_d D2M[m][d] psi[d][e]  -- direction -> moment reduction
 template <typename real>
 cudaError_t launch_reduce_moments(const real* psi, const real* d2m_t, real* phi, int n_dir,
-                                  int n_mom, long n_dofs, cudaStream_t s, long len = -1);
+                                  int n_mom, long n_dofs, cudaStream_t s, long len = -1, const double* xc = nullptr,
+                                  double* y = nullptr);
 
 // ------------------------------------------------------------ vector kernels
 template <typename real>

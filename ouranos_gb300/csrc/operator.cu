@@ -625,23 +625,24 @@ int sweep_prepare(ouranos_rt* rt, const real* src, const real* iso, const real* 
 
 // phi = D2M psi (the moment reduction after a sweep); phi is float for the
 // FP32 sweep, double for the FP64 and double-float sweeps
-// The double-float reductions can write the Apply's y = x - phi in phi's
-// place (one rounding, as the combine kernel): one kernel and one pass over
-// phi less per Apply
+// The double-float reductions and the FP32 one can write the Apply's y = x - phi
+// in phi's place (one rounding, as the combine kernel): one kernel and one pass
+// over phi less per Apply
 bool fused_combine(const ouranos_rt* rt) {
+  if (rt->precision != OURANOS_FP64) return rt->fp32_contract != OURANOS_FP32_CONTRACT_TENSOR;
   return df64_sweep(rt) && (rt->fp64_contract == OURANOS_FP64_DF64_SWEEP_TC ? rt->oz.npad > 0 : rt->sym.n_class > 0);
 }
 
 template <typename real>
 int sweep_reduce(ouranos_rt* rt, const real* psi, void* phi, long e0 = 0, long len = -1, const double* xc = nullptr) {
   // dofs [e0, e0 + len): psi and phi move by e0, their row stride stays n_dofs;
-  // with xc (fused_combine only), phi receives xc - phi
+  // with xc (fused_combine only), phi receives xc - phi, in FP64 whatever the sweep
   const long nd = rt->n_dofs;
   if (len < 0) len = nd;
   psi += e0;
   double* phi64 = (double*)phi + e0;
   if (xc) {
-    if (!std::is_same<real, df64>::value || !fused_combine(rt)) return bad(rt, "no fused combination here");
+    if (std::is_same<real, double>::value || !fused_combine(rt)) return bad(rt, "no fused combination here");
     xc += e0;
   }
   if (std::is_same<real, df64>::value && rt->fp64_contract == OURANOS_FP64_DF64_SWEEP_TC)
@@ -668,8 +669,8 @@ int sweep_reduce(ouranos_rt* rt, const real* psi, void* phi, long e0 = 0, long l
                         rt->wait_limit_ns, rt->stream, len),
        "moment reduction");
   else
-    CU(launch_reduce_moments<float>((const float*)psi, rt->d_d2m32.as<float>(), (float*)phi + e0, rt->n_dir,
-                                    rt->n_mom, nd, rt->stream, len),
+    CU(launch_reduce_moments<float>((const float*)psi, rt->d_d2m32.as<float>(), xc ? nullptr : (float*)phi + e0,
+                                    rt->n_dir, rt->n_mom, nd, rt->stream, len, xc, xc ? phi64 : nullptr),
        "moment reduction");
   return OURANOS_OK;
 }
@@ -1010,7 +1011,10 @@ void nominal_tiling(const ouranos_rt* rt, int& wx, int& wy, int& lpc) {
 int rt_apply_device(ouranos_rt* rt, const double* x, double* y) {
   OK_OR_RETURN(build_source(rt, x, nullptr, df64_sweep(rt)));
   if (fused_combine(rt)) {  // the reduction writes y = x - phi
-    OK_OR_RETURN(run_sweep<df64>(rt, rt->d_src64.as<df64>(), nullptr, nullptr, y, x));
+    if (rt->precision == OURANOS_FP64)
+      OK_OR_RETURN(run_sweep<df64>(rt, rt->d_src64.as<df64>(), nullptr, nullptr, y, x));
+    else
+      OK_OR_RETURN(run_sweep<float>(rt, rt->d_src32.as<float>(), nullptr, nullptr, y, x));
     rt->last_kernels += 1;  // the scattering source
     return OURANOS_OK;
   }
@@ -1062,6 +1066,8 @@ int rt_batch_prepare(ouranos_rt* rt, const double* x, SweepArgs<float>* a, int* 
 int rt_batch_finish(ouranos_rt* rt, const double* x, double* y, bool sources) {
   if (rt->precision == OURANOS_FP64)
     OK_OR_RETURN(sweep_reduce<double>(rt, rt->d_psi.as<double>(), rt->d_phi64.p));
+  else if (!sources && fused_combine(rt))
+    return sweep_reduce<float>(rt, rt->d_psi.as<float>(), y, 0, -1, x);
   else
     OK_OR_RETURN(sweep_reduce<float>(rt, rt->d_psi.as<float>(), rt->d_phi32.p));
   return sources ? phi_combine(rt, nullptr, y, 0.0, 1.0) : phi_combine(rt, x, y, 1.0, -1.0);

@@ -8,6 +8,7 @@
 
 #include "df64.cuh"
 #include "internal.h"
+#include "pack2.cuh"
 
 namespace ouranos {
 namespace {
@@ -115,7 +116,7 @@ __global__ void combine_kernel(const double* x, const real* phi, double* y, long
                                double sp) {
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < len;
        e += (long)gridDim.x * blockDim.x)
-    y[e] = (x ? sx * x[e] : 0.0) + sp * (double)phi[e];
+    y[e] = (x ? sx * x[e] : 0.0) + sp * real_to_double(phi[e]);
 }
 
 // y = sx x + sp phi on rows x len elements of row stride `stride` (one dof
@@ -266,6 +267,8 @@ __global__ void __launch_bounds__(kBlock) dots_final_kernel(const double* partia
 // axis with the coefficient table in shared memory.
 //   expand:  q[d][e] (+)= sum_{m<nm} m2d[d*ld + m] T[m][e] (+ iso[e])
 //   reduce:  phi[m][e]   = sum_d d2m_t[d*ld + m] psi[d][e],  m < nm
+//            or, with xc, y[m][e] = xc[m][e] - that sum (the Apply's combination: one
+//            kernel and a pass over phi less: FP32 128^3 LS S8 868 + 100 -> 932 us)
 template <typename real, int NM>
 __global__ void expand_kernel(const real* __restrict__ T, const real* __restrict__ iso,
                               const real* __restrict__ m2d, int ld, real* __restrict__ q,
@@ -292,7 +295,8 @@ __global__ void expand_kernel(const real* __restrict__ T, const real* __restrict
 
 template <typename real, int NM>
 __global__ void reduce_kernel(const real* __restrict__ psi, const real* __restrict__ d2m_t, int ld,
-                              real* __restrict__ phi, int n_dir, int nm, long n_dofs, long len) {
+                              real* __restrict__ phi, int n_dir, int nm, long n_dofs, long len, const double* xc,
+                              double* y) {
   extern __shared__ unsigned char smem_raw[];
   real* sm = reinterpret_cast<real*>(smem_raw);
   for (int k = threadIdx.x; k < n_dir * nm; k += blockDim.x) sm[k] = d2m_t[(k / nm) * ld + k % nm];
@@ -310,7 +314,11 @@ __global__ void reduce_kernel(const real* __restrict__ psi, const real* __restri
     }
 #pragma unroll
     for (int m = 0; m < NM; ++m)
-      if (m < nm) phi[(size_t)m * n_dofs + e] = acc[m];
+      if (m < nm) {
+        const size_t i = (size_t)m * n_dofs + e;
+        if (xc) y[i] = xc[i] - (sizeof(real) == 4 ? f64_from_f32((float)acc[m]) : (double)acc[m]);
+        else phi[i] = acc[m];
+      }
   }
 }
 
@@ -760,29 +768,31 @@ template cudaError_t launch_expand_source<float>(const float*, const float*, con
 
 template <typename real>
 cudaError_t launch_reduce_moments(const real* psi, const real* d2m_t, real* phi, int n_dir,
-                                  int n_mom, long n_dofs, cudaStream_t s, long len) {
+                                  int n_mom, long n_dofs, cudaStream_t s, long len, const double* xc, double* y) {
   if (len < 0) len = n_dofs;
   for (int m0 = 0; m0 < n_mom; m0 += 16) {
     const int nm = n_mom - m0 < 16 ? n_mom - m0 : 16;
     const size_t sh = sizeof(real) * (size_t)n_dir * nm;
-    real* ph = phi + (size_t)m0 * n_dofs;
+    real* ph = xc ? nullptr : phi + (size_t)m0 * n_dofs;
+    const double* xm = xc ? xc + (size_t)m0 * n_dofs : nullptr;
+    double* ym = xc ? y + (size_t)m0 * n_dofs : nullptr;
     if (nm <= 1)
-      reduce_kernel<real, 1><<<resident_grid(reduce_kernel<real, 1>, len, sh), kBlock, sh, s>>>(psi, d2m_t + m0, n_mom, ph, n_dir, nm, n_dofs, len);
+      reduce_kernel<real, 1><<<resident_grid(reduce_kernel<real, 1>, len, sh), kBlock, sh, s>>>(psi, d2m_t + m0, n_mom, ph, n_dir, nm, n_dofs, len, xm, ym);
     else if (nm <= 4)
-      reduce_kernel<real, 4><<<resident_grid(reduce_kernel<real, 4>, len, sh), kBlock, sh, s>>>(psi, d2m_t + m0, n_mom, ph, n_dir, nm, n_dofs, len);
+      reduce_kernel<real, 4><<<resident_grid(reduce_kernel<real, 4>, len, sh), kBlock, sh, s>>>(psi, d2m_t + m0, n_mom, ph, n_dir, nm, n_dofs, len, xm, ym);
     else if (nm <= 10)
-      reduce_kernel<real, 10><<<resident_grid(reduce_kernel<real, 10>, len, sh), kBlock, sh, s>>>(psi, d2m_t + m0, n_mom, ph, n_dir, nm, n_dofs, len);
+      reduce_kernel<real, 10><<<resident_grid(reduce_kernel<real, 10>, len, sh), kBlock, sh, s>>>(psi, d2m_t + m0, n_mom, ph, n_dir, nm, n_dofs, len, xm, ym);
     else
-      reduce_kernel<real, 16><<<resident_grid(reduce_kernel<real, 16>, len, sh), kBlock, sh, s>>>(psi, d2m_t + m0, n_mom, ph, n_dir, nm, n_dofs, len);
+      reduce_kernel<real, 16><<<resident_grid(reduce_kernel<real, 16>, len, sh), kBlock, sh, s>>>(psi, d2m_t + m0, n_mom, ph, n_dir, nm, n_dofs, len, xm, ym);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
 template cudaError_t launch_reduce_moments<double>(const double*, const double*, double*, int, int,
-                                                   long, cudaStream_t, long);
+                                                   long, cudaStream_t, long, const double*, double*);
 template cudaError_t launch_reduce_moments<float>(const float*, const float*, float*, int, int,
-                                                  long, cudaStream_t, long);
+                                                  long, cudaStream_t, long, const double*, double*);
 
 // Arithmetic of the per-cell scattering source: FP32 for the FP32 sweep,
 // double-float for the FP64 sweep's pair storage
@@ -792,7 +802,7 @@ template <>
 struct SrcArith<float> {
   using T = float;
   using Acc = float;
-  __device__ static T from(double v) { return (float)v; }
+  __device__ static T from(double v) { return f32_from_f64(v); }
   __device__ static Acc zero() { return 0.f; }
   __device__ static void fma(Acc& a, T u, T v) { a = __fmaf_rn(u, v, a); }
   __device__ static Acc prod(T u, T v) { return __fmul_rn(u, v); }
@@ -817,45 +827,73 @@ struct SrcArith<df64> {
 // other-group terms: the cell's N values of x are converted once and the
 // N x N mass-matrix products run on the FP32 pipes.  (One thread per output
 // in FP64 spent N FP64 multiply-adds per value on GB300's 1/64-rate FP64
-// pipe.)  Cells are the fastest index, so a warp reads and writes 32 * N
-// consecutive values.
+// pipe.)  A warp's 32 cells are consecutive in memory: it reads and writes them
+// as one run, through a shared slot (rows of odd length: every lane its own
+// bank), where each lane keeps its cell.  A lane on its own cell touched 32
+// sectors an instruction, a third of each at a time.  With that and the conversions
+// off the FP64 pipe: FP32 128^3 Q1 80 -> 70 us, 256^2 Q2 with ten moments 63 -> 48.
+constexpr int kCellWarps = 4;  // (2 / 1 warps: 67 / 89 us in FP32, 95 / 114 against 92 for 3-D Q2)
 template <typename real, int N>
-__global__ void __launch_bounds__(kBlock) scatter_cell_kernel(const double* __restrict__ x, real* __restrict__ src,
-                                                              const double* __restrict__ M,
-                                                              const double* __restrict__ sscale,
-                                                              const int* __restrict__ material, long n_cells,
-                                                              int n_mom, long n_dofs) {
+__global__ void __launch_bounds__(32 * kCellWarps) scatter_cell_kernel(const double* __restrict__ x,
+                                                                       real* __restrict__ src,
+                                                                       const double* __restrict__ M,
+                                                                       const double* __restrict__ sscale,
+                                                                       const int* __restrict__ material, long n_cells,
+                                                                       int n_mom, long n_dofs) {
   using A = SrcArith<real>;
-  __shared__ typename A::T sM[N * N];
+  using T = typename A::T;
+  constexpr int ST = N | 1;
+  __shared__ T sM[N * N], slots[kCellWarps][32 * ST];
   for (int k = threadIdx.x; k < N * N; k += blockDim.x) sM[k] = A::from(M[k]);
   __syncthreads();
-  const long total = (long)n_mom * n_cells;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
-    const long c = t % n_cells;
-    const int m = (int)(t / n_cells);
-    const double* xc = x + (size_t)m * n_dofs + c * N;
-    typename A::T xv[N];
+  const int lane = threadIdx.x & 31;
+  T* slot = slots[threadIdx.x >> 5];
+  const long runs = (n_cells + 31) / 32, total = runs * n_mom;
+  for (long t = blockIdx.x * (long)kCellWarps + (threadIdx.x >> 5); t < total; t += (long)gridDim.x * kCellWarps) {
+    const int m = (int)(t / runs);
+    const long c0 = (t - m * runs) * 32;
+    const int cells = n_cells - c0 < 32 ? (int)(n_cells - c0) : 32;
+    const double* xc = x + (size_t)m * n_dofs + c0 * N;
+    real* out = src + (size_t)m * n_dofs + c0 * N;
+    T sc = T(0.f);
+    if (lane < cells) sc = A::from(__ldg(sscale + (size_t)__ldg(material + c0 + lane) * n_mom + m));
 #pragma unroll
-    for (int j = 0; j < N; ++j) xv[j] = A::from(__ldg(xc + j));
-    const typename A::T sc = A::from(__ldg(sscale + (size_t)material[c] * n_mom + m));
-    real* out = src + (size_t)m * n_dofs + c * N;
-#pragma unroll 1
-    for (int i = 0; i < N; ++i) {
-      typename A::Acc acc = A::prod(sM[i * N], xv[0]);
-#pragma unroll
-      for (int j = 1; j < N; ++j) A::fma(acc, sM[i * N + j], xv[j]);
-      out[i] = A::out(acc, sc);
+    for (int j = 0; j < N; ++j) {
+      const int u = lane + 32 * j;
+      if (u < cells * N) slot[u / N * ST + u % N] = A::from(__ldg(xc + u));
     }
+    __syncwarp();
+    if (lane < cells) {
+      T* own = slot + lane * ST;
+      T xv[N];
+#pragma unroll
+      for (int j = 0; j < N; ++j) xv[j] = own[j];
+#pragma unroll 1
+      for (int i = 0; i < N; ++i) {
+        typename A::Acc acc = A::prod(sM[i * N], xv[0]);
+#pragma unroll
+        for (int j = 1; j < N; ++j) A::fma(acc, sM[i * N + j], xv[j]);
+        own[i] = A::out(acc, sc);
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const int u = lane + 32 * j;
+      if (u < cells * N) out[u] = slot[u / N * ST + u % N];
+    }
+    __syncwarp();
   }
 }
 
 template <typename real, int N>
 static cudaError_t scatter_cell(const double* x, real* src, const double* M, const double* sscale,
                                 const int* material, long n_cells, int n_mom, long n_dofs, cudaStream_t s) {
-  long g = ((long)n_mom * n_cells + kBlock - 1) / kBlock;
-  if (g > 152L * 8) g = 152L * 8;  // each block converts the mass matrix once
-  scatter_cell_kernel<real, N><<<(int)(g < 1 ? 1 : g), kBlock, 0, s>>>(x, src, M, sscale, material, n_cells, n_mom,
-                                                                       n_dofs);
+  // a block's share of the mass matrix's conversion is small: no cap on the blocks
+  // (8 an SM: 89 us instead of 70 for FP32 128^3)
+  const long g = std::min(((n_cells + 31) / 32 * n_mom + kCellWarps - 1) / kCellWarps, 1L << 30);
+  scatter_cell_kernel<real, N><<<(int)(g < 1 ? 1 : g), 32 * kCellWarps, 0, s>>>(x, src, M, sscale, material, n_cells,
+                                                                               n_mom, n_dofs);
   return cudaGetLastError();
 }
 template <typename real>
@@ -976,14 +1014,17 @@ namespace {
 template <typename real, int N>
 __global__ void __launch_bounds__(256) angular_source_kernel(real* __restrict__ q, const float* __restrict__ psi,
                                                              const double* __restrict__ M, double inv_vdt,
-                                                             long n_cells, int n_dir) {
+                                                             long n_cells, int n_dir, float minus_zero) {
   constexpr bool F32 = sizeof(real) == 4;
   __shared__ df64 sd[N * N];
   __shared__ float sf[N * N];
+  __shared__ Pk<df64>::P sp[(N + 1) / 2 * N];  // rows 2k and 2k + 1
   for (int k = threadIdx.x; k < N * N; k += blockDim.x) {
     const double m = inv_vdt * M[k];
     sd[k] = df64_from(m);
     sf[k] = (float)m;
+    const int i = k / N, j = k % N;
+    if (i % 2 == 0) sp[i / 2 * N + j] = Pk<df64>::make(df64_from(m), i + 1 < N ? df64_from(inv_vdt * M[k + N]) : df64(0.f));
   }
   __syncthreads();
   const long total = (long)n_dir * n_cells;
@@ -1004,6 +1045,25 @@ __global__ void __launch_bounds__(256) angular_source_kernel(real* __restrict__ 
       for (int j = 0; j < N; ++j) p[j] = pc[j];
     }
     real* qc = q + t * N;
+    // pairs, N even: two rows at a time in packed FP32 operations, 16 bytes a load and
+    // store (8 bytes a lane and row touched every sector four times; rate-bound by the
+    // 12 operations of a multiply-add, 80 us of LS S8 40x36x33, where 164 us became 119)
+    if constexpr (std::is_same<real, df64>::value && N % 2 == 0) {
+      using K = Pk<df64>;
+      const f2 z = f2_make(minus_zero, minus_zero);
+      K::Op pv[N];
+#pragma unroll
+      for (int j = 0; j < N; ++j) pv[j] = K::op(K::make(df64(p[j]), df64(p[j])));
+#pragma unroll 1
+      for (int i = 0; i < N; i += 2) {
+        unsigned char* at = reinterpret_cast<unsigned char*>(qc + i);
+        K::Acc acc = K::from(K::array_load(at));
+#pragma unroll
+        for (int j = 0; j < N; ++j) K::fma(acc, sp[i / 2 * N + j], pv[j], z);
+        K::array_put(at, K::result(acc));
+      }
+      continue;
+    }
 #pragma unroll 1
     for (int i = 0; i < N; ++i) {
       if constexpr (F32) {
@@ -1030,7 +1090,7 @@ cudaError_t launch_angular_source(real* q, const float* psi, const double* cell_
   switch (n) {
 #define CASE(NN)                                                                                             \
   case NN:                                                                                                   \
-    angular_source_kernel<real, NN><<<grid, 256, 0, s>>>(q, psi, cell_mass, inv_vdt, n_cells, n_dir);         \
+    angular_source_kernel<real, NN><<<grid, 256, 0, s>>>(q, psi, cell_mass, inv_vdt, n_cells, n_dir, -0.f);    \
     break;
     CASE(4) CASE(8) CASE(9) CASE(16) CASE(25) CASE(27)
 #undef CASE
