@@ -8,6 +8,10 @@
 //                 that class (class = dimension, FE order, fused-moment form),
 //                 warps taking (problem, task) pairs in ticket order,
 //   per problem   the moment reduction and y = x - phi.
+// The kernels of one problem do not fill the GPU: the problems' prepare and finish
+// work goes to side streams, the classes' sweeps run side by side, and a problem is
+// finished as soon as its class's sweep is done; the batch's stream waits for all
+// (16 2-D problems of 32^2 to 256^2, FP32: 2017 -> 1717 us).
 // The edge-word epoch lives in device memory and is advanced by a kernel, the
 // tickets are reset by memset nodes, and every pointer is fixed once the
 // buffers have been sized, so the whole Apply is captured into a CUDA graph on
@@ -37,6 +41,7 @@ constexpr int kStatus = kMaxClasses;      // d_ctrl[kStatus]: sticky timeout fla
 constexpr int kEpoch = kMaxClasses + 1;   // d_ctrl[kEpoch]: edge-word epoch
 constexpr size_t kMaxGraphs = 64;         // captured Apply graphs kept per batch
 constexpr size_t kMaxTicketMaps = 256;
+constexpr int kSides = 8;                 // side streams
 
 struct TicketMap {
   // classes present in the set: (dim, p1, fm, form), first ticket-map entry, count
@@ -59,6 +64,10 @@ struct ouranos_batch {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_in = nullptr, ev0 = nullptr, ev1 = nullptr;
+  // side streams, the events that order them after and before the batch's stream,
+  // and the sweeps' ends
+  cudaStream_t side[kSides] = {};
+  cudaEvent_t ev_fork = nullptr, ev_side[kSides] = {}, ev_sweep[kMaxClasses] = {};
   std::string err;
   int sms = 0;
   std::vector<ouranos_rt*> rt;
@@ -161,6 +170,30 @@ int ticket_map(ouranos_batch* b, const std::vector<char>& mask, TicketMap** out)
   return OURANOS_OK;
 }
 
+// Order the side streams after the work queued on the batch's stream, and the
+// batch's stream after theirs.
+int fork_sides(ouranos_batch* b) {
+  BC(cudaEventRecord(b->ev_fork, b->stream), "order");
+  for (cudaStream_t s : b->side) BC(cudaStreamWaitEvent(s, b->ev_fork, 0), "order");
+  return OURANOS_OK;
+}
+int join_sides(ouranos_batch* b) {
+  for (int k = 0; k < kSides; ++k) {
+    BC(cudaEventRecord(b->ev_side[k], b->side[k]), "order");
+    BC(cudaStreamWaitEvent(b->stream, b->ev_side[k], 0), "order");
+  }
+  return OURANOS_OK;
+}
+// f() with problem p's handle on stream s
+template <typename F>
+int on_stream(ouranos_batch* b, int p, cudaStream_t s, F f) {
+  cudaStream_t keep = b->rt[p]->stream;
+  b->rt[p]->stream = s;
+  const int rc = f();
+  b->rt[p]->stream = keep;
+  return member(b, p, rc);
+}
+
 // Enqueue one batched Apply of the problems in `mask` (no synchronisation):
 // y = x - D L^-1 M2D S x per slice, or with sources, y = D L^-1 (q + inflow).
 template <typename real>
@@ -172,15 +205,24 @@ int apply_body(ouranos_batch* b, const std::vector<char>& mask, bool sources, Ti
   const double* X = b->d_X.as<double>();
   double* Y = b->d_Y.as<double>();
   int* ctrl = b->d_ctrl.as<int>();
-  for (size_t p = 0; p < b->rt.size(); ++p) {
-    if (!mask[p]) continue;
-    int fm = 0;
-    BR(member(b, (int)p, rt_batch_prepare(b->rt[p], sources ? nullptr : X + b->off[p], &h_args[p], &fm,
-                                          sources)));
-    if (fm != b->fm[p]) return bbad(b, "fused-moment form changed");
-    h_args[p].ticket = ctrl;
-    h_args[p].status = ctrl + kStatus;
-  }
+  const int P = (int)b->rt.size();
+  BR(fork_sides(b));
+  auto prepare = [&]() -> int {
+    for (int p = 0; p < P; ++p) {
+      if (!mask[p]) continue;
+      int fm = 0;
+      BR(on_stream(b, p, b->side[p % kSides], [&] {
+        return rt_batch_prepare(b->rt[p], sources ? nullptr : X + b->off[p], &h_args[p], &fm, sources);
+      }));
+      if (fm != b->fm[p]) return bbad(b, "fused-moment form changed");
+      h_args[p].ticket = ctrl;
+      h_args[p].status = ctrl + kStatus;
+    }
+    return OURANOS_OK;
+  };
+  const int rp = prepare();
+  BR(join_sides(b));  // (whatever was queued, also after a failure)
+  BR(rp);
   BC(cudaMemcpyAsync(d_args.p, h_args, sizeof(SweepArgs<real>) * b->rt.size(), cudaMemcpyHostToDevice,
                      b->stream),
      "sweep arguments");
@@ -191,20 +233,42 @@ int apply_body(ouranos_batch* b, const std::vector<char>& mask, bool sources, Ti
   BC(cudaStreamIsCapturing(b->stream, &cap), "capture status");
   const unsigned rec = cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
   BC(cudaEventRecordWithFlags(b->ev0, b->stream, rec), "event");
-  for (size_t c = 0; c < tm->cls.size(); ++c) {
-    const TicketMap::Cls& k = tm->cls[c];
-    const int grid = (int)std::min<long>((k.count + 3) / 4, (long)std::max(1, b->sms * 8));
-    BC(launch_sweep_batch<real>(k.dim, k.p1, k.fm, k.lpc, k.grouped, sources, d_args.as<SweepArgs<real>>(),
-                                tm->d.as<int2>() + k.first, (int)k.count, ctrl + c, ctrl + kStatus,
-                                (const unsigned*)(ctrl + kEpoch), grid, 128, b->stream),
-       "batched sweep");
-  }
-  BC(cudaEventRecordWithFlags(b->ev1, b->stream, rec), "event");
-  for (size_t p = 0; p < b->rt.size(); ++p) {
-    if (!mask[p]) continue;
-    BR(member(b, (int)p, rt_batch_finish(b->rt[p], sources ? nullptr : X + b->off[p], Y + b->off[p], sources)));
-  }
-  return OURANOS_OK;
+  BR(fork_sides(b));
+  // sweeps on the first streams, the problems' finishes on the others
+  const int ns = (int)std::min<size_t>(tm->cls.size(), kSides / 2), nf = kSides - ns;
+  auto sweeps = [&]() -> int {
+    for (size_t c = 0; c < tm->cls.size(); ++c) {
+      const TicketMap::Cls& k = tm->cls[c];
+      cudaStream_t s = b->side[c % ns];
+      const int grid = (int)std::min<long>((k.count + 3) / 4, (long)std::max(1, b->sms * 8));
+      BC(launch_sweep_batch<real>(k.dim, k.p1, k.fm, k.lpc, k.grouped, sources, d_args.as<SweepArgs<real>>(),
+                                  tm->d.as<int2>() + k.first, (int)k.count, ctrl + c, ctrl + kStatus,
+                                  (const unsigned*)(ctrl + kEpoch), grid, 128, s),
+         "batched sweep");
+      BC(cudaEventRecord(b->ev_sweep[c], s), "order");
+      BC(cudaStreamWaitEvent(b->stream, b->ev_sweep[c], 0), "order");
+    }
+    BC(cudaEventRecordWithFlags(b->ev1, b->stream, rec), "event");
+    int next = 0;
+    for (size_t c = 0; c < tm->cls.size(); ++c) {
+      const TicketMap::Cls& k = tm->cls[c];
+      for (int p = 0; p < P; ++p) {
+        const ouranos_rt* r = b->rt[p];
+        if (!mask[p] || r->dim != k.dim || r->p1 != k.p1 || b->fm[p] != k.fm || r->lpc != k.lpc ||
+            r->grouped != k.grouped)
+          continue;
+        cudaStream_t s = b->side[ns + next++ % nf];
+        BC(cudaStreamWaitEvent(s, b->ev_sweep[c], 0), "order");
+        BR(on_stream(b, p, s, [&] {
+          return rt_batch_finish(b->rt[p], sources ? nullptr : X + b->off[p], Y + b->off[p], sources);
+        }));
+      }
+    }
+    return OURANOS_OK;
+  };
+  const int rs = sweeps();
+  BR(join_sides(b));
+  return rs;
 }
 
 int apply_any(ouranos_batch* b, int precision, const std::vector<char>& mask, bool sources, TicketMap* tm) {
@@ -366,7 +430,10 @@ int ouranos_batch_create(const ouranos_problem_desc* descs, int count, int devic
     if (r->device != b->device) return bbad(b, "all problems of a batch must be on one device");
   cudaSetDevice(b->device);
   BC(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "stream");
-  BC(cudaEventCreateWithFlags(&b->ev_in, cudaEventDisableTiming), "event");
+  for (cudaStream_t& s : b->side) BC(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
+  for (cudaEvent_t* e : {&b->ev_in, &b->ev_fork}) BC(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "event");
+  for (cudaEvent_t& e : b->ev_side) BC(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+  for (cudaEvent_t& e : b->ev_sweep) BC(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
   BC(cudaEventCreate(&b->ev0), "event");
   BC(cudaEventCreate(&b->ev1), "event");
   BC(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device), "device query");
@@ -412,7 +479,17 @@ int ouranos_batch_destroy(ouranos_batch* b) {
     if (b->h_args64[s]) cudaFreeHost(b->h_args64[s]);
     if (b->h_args32[s]) cudaFreeHost(b->h_args32[s]);
   }
-  if (b->ev_in) cudaEventDestroy(b->ev_in);
+  for (cudaStream_t s : b->side)
+    if (s) {
+      cudaStreamSynchronize(s);
+      cudaStreamDestroy(s);
+    }
+  for (cudaEvent_t e : {b->ev_in, b->ev_fork})
+    if (e) cudaEventDestroy(e);
+  for (cudaEvent_t e : b->ev_side)
+    if (e) cudaEventDestroy(e);
+  for (cudaEvent_t e : b->ev_sweep)
+    if (e) cudaEventDestroy(e);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->stream) cudaStreamDestroy(b->stream);
