@@ -123,6 +123,8 @@ struct SweepArgs {
   int lpc;                     // lanes per cell: 1, 2 (cells of 9 or more dofs), or 32 (one warp
                                // per cell, sweep_wide.cuh; tiling 1 x 1 x 1, expanded source)
   int grouped;                 // 1: the default form, lpc lanes per cell (sweep_group.cuh)
+  int n_queues;                // more than 1 (grouped, lpc > 1): tasks come in queues, queue k's entries
+  const int* queue_first;      // [queue_first[k], queue_first[k + 1]), each with a counter of its own at ticket[k]
   float minus_zero;            // -0, an addend the compiler does not know (pack2.cuh)
   // one lane per cell (sweep_lane.cuh): the materials of the columns, four planes
   // to a word, [sweep direction][plane / 4][column] (NULL: more than 256
@@ -462,6 +464,8 @@ struct ouranos_rt {
   bool grouped = false;                // the default form (sweep_group.cuh); wx, wy, lpc are its own
   int tiles_x = 0, tiles_y = 0, n_groups_dir = 0, n_tasks = 0;
   std::vector<int> dir_class_h;
+  ouranos::DevBuf d_queue_tasks, d_queue_first;  // tasks by |Omega| class (SweepArgs::queue_first)
+  int n_queues = 1;
   std::vector<double> class_abs_omega;  // [n_dir_class][3]
   int n_dir_class = 0;
   std::vector<double> sigma_class_value; // per sigma_t class

@@ -209,6 +209,8 @@ int apply_noalloc(ouranos_rt* rt, unsigned char* base, const Layout& L, bool exp
   a.kd = rt->kd;
   a.lpc = rt->lpc;
   a.grouped = rt->grouped;
+  a.n_queues = 1;
+  a.queue_first = nullptr;
   a.cls4 = rt->cls4_ok ? rt->d_cls4.as<unsigned>() : nullptr;
   a.face_group = tbl<real>(rt->d_fgroup64, rt->d_fgroup32, rt->d_fgroupdf);
   a.minus_zero = -0.f;

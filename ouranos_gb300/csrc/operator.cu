@@ -197,6 +197,19 @@ int build_symmetry(ouranos_rt* rt) {
 // ------------------------------------------------------------------ schedule
 // Directions of one octant (same sign pattern) are grouped kd at a time; each
 // group crosses the transverse tiles in dependency order.
+// Task counters of the queues in the control block, after the ticket and the status
+constexpr int kQueueTickets = 2, kMaxQueues = 48;
+
+// Whether the inverse tables of all |Omega| classes are more than an SM's L1 keeps
+// beside the slots, so that its warps should work on one class at a time.  Apply, us,
+// one queue / a queue per class / with 132 KB of L1 kept for it (kGroupKeepKb):
+// 3-D Q3 20x17x23 LS S4, two materials (32 KB a table) 1342 / 1294 / 1167, the larger L1
+// alone 1396; 3-D Q2 37x29x41 LS S6 (6 KB a table) 2152 / 2102 / 2108.
+bool tables_spill(const ouranos_rt* rt, size_t real_bytes) {
+  const size_t table = real_bytes * rt->n * rt->n * rt->sigma_class_value.size();
+  return rt->n_queues > 1 && table * rt->n_dir_class > (64u << 10);
+}
+
 int build_schedule(ouranos_rt* rt) {
   const int dim = rt->dim;
   const int NX = rt->nx[0], NY = dim == 3 ? rt->nx[1] : 1, NS = rt->nx[dim - 1];
@@ -231,6 +244,19 @@ int build_schedule(ouranos_rt* rt) {
       }
   rt->n_tasks = (int)tasks.size();
   OK_OR_RETURN(upload(rt, rt->d_tasks, tasks, "tasks"));
+  // the same tasks by |Omega| class, each class's in the order above (tables_spill)
+  rt->n_queues = rt->grouped && rt->lpc > 1 && rt->n_dir_class <= kMaxQueues ? rt->n_dir_class : 1;
+  if (rt->n_queues > 1) {
+    std::vector<int2> by_class;
+    std::vector<int> first(1, 0);
+    for (int c = 0; c < rt->n_dir_class; ++c) {
+      for (const int2& t : tasks)
+        if (rt->dir_class_h[gdirs[t.x]] == c) by_class.push_back(t);
+      first.push_back((int)by_class.size());
+    }
+    OK_OR_RETURN(upload(rt, rt->d_queue_tasks, by_class, "tasks"));
+    OK_OR_RETURN(upload(rt, rt->d_queue_first, first, "tasks"));
+  }
   OK_OR_RETURN(upload(rt, rt->d_group_dirs, gdirs, "group dirs"));
   OK_OR_RETURN(upload(rt, rt->d_group_flip, gflip, "group flips"));
   // control block: [0] ticket, [1] status (the rest is spare)
@@ -570,6 +596,8 @@ int sweep_prepare(ouranos_rt* rt, const real* src, const real* iso, const real* 
   a.kd = rt->kd;
   a.lpc = rt->lpc;
   a.grouped = rt->grouped;
+  a.n_queues = 1;
+  a.queue_first = nullptr;
   a.cls4 = rt->cls4_ok ? rt->d_cls4.as<unsigned>() : nullptr;
   a.face_group = table<real>(rt->d_fgroup64, rt->d_fgroup32, rt->d_fgroupdf);
   a.minus_zero = -0.f;
@@ -686,11 +714,17 @@ int sweep_launch(ouranos_rt* rt, SweepArgs<real>& a, int fm) {
   int* ctrl = rt->d_ctrl.as<int>();
   a.ticket = ctrl;
   a.status = ctrl + 1;
-  // ticket -> 0.  The status word [1] is sticky: it is cleared at the start of
+  if (tables_spill(rt, sizeof(real))) {
+    a.n_queues = rt->n_queues;
+    a.queue_first = rt->d_queue_first.as<int>();
+    a.tasks = rt->d_queue_tasks.as<int2>();
+    a.ticket = ctrl + kQueueTickets;
+  }
+  // tickets -> 0.  The status word [1] is sticky: it is cleared at the start of
   // each C-ABI call (clear_status), so a timeout inside a solve (a sweep's
   // dependency wait, bit 1; a diffusion-solve barrier, bit 2) is seen at its
   // end and every later sweep of that call exits at once.
-  CU(cudaMemsetAsync(ctrl, 0, sizeof(int), rt->stream), "reset sweep control");
+  CU(cudaMemsetAsync(a.ticket, 0, sizeof(int) * a.n_queues, rt->stream), "reset sweep control");
   int sms = 0;
   CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, rt->device), "device query");
   const int block = 128;

@@ -625,15 +625,36 @@ template <typename real, int DIM, int P1, int FM, int H>
 __global__ void __launch_bounds__(128) sweep_group_kernel(const __grid_constant__ SweepArgs<real> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr unsigned FULL = 0xffffffffu;
+  // With queues, an SM starts on one |Omega| class, whose tables its L1 then holds, and
+  // goes on to the next when that has no tasks left.  Every queue is in dependency
+  // order and a class's tasks wait on none of another's, so any warp may take the
+  // head of any queue.
+  int queue = 0, left = a.n_queues;
+  if (left > 1) {
+    unsigned sm;
+    asm("mov.u32 %0, %%smid;" : "=r"(sm));
+    queue = (int)(sm % (unsigned)left);
+  }
   for (;;) {
     int task = 0, stop = 0;
     if ((threadIdx.x & 31) == 0) {
-      task = atomicAdd(a.ticket, 1);
+      task = atomicAdd(a.ticket + queue, 1);
       stop = *(volatile int*)a.status;
     }
     task = __shfl_sync(FULL, task, 0);
     stop = __shfl_sync(FULL, stop, 0);
-    if (task >= a.n_tasks || stop) return;
+    if (stop) return;
+    int count = a.n_tasks;
+    if (a.n_queues > 1) {
+      const int first = a.queue_first[queue];
+      count = a.queue_first[queue + 1];
+      task += first;
+    }
+    if (task >= count) {
+      if (--left == 0) return;
+      queue = queue + 1 == a.n_queues ? 0 : queue + 1;
+      continue;
+    }
     sweep_group_task<real, DIM, P1, FM, H>(a, task, smem_raw);
   }
 }
@@ -697,8 +718,10 @@ __global__ void __launch_bounds__(128) sweep_group_batch_kernel(const SweepArgs<
 
 // L1 kept beside the resident blocks, for the inverse tables of the running
 // directions: the sources stream past it (16-byte cp.async.cg), and 28, 64 and
-// 112 KB measured the same within the spread
-constexpr int kGroupKeepKb = 64;
+// 112 KB measured the same within the spread; more where an SM's warps share one
+// class's tables (3-D Q3 20x17x23, us, 64 / 100 / 132 / 164 KB: 1294 / 1193 / 1167 / 1170;
+// 3-D Q2 37x29x41: 2102 / 2095 / 2108 / 2400)
+constexpr int kGroupKeepKb = 64, kQueueKeepKb = 132;
 
 template <typename real, int DIM, int P1, int FM, int H>
 cudaError_t launch_group_fm(const SweepArgs<real>& a, int grid, int block, cudaStream_t s) {
@@ -707,7 +730,7 @@ cudaError_t launch_group_fm(const SweepArgs<real>& a, int grid, int block, cudaS
   const size_t warps = block / 32, smem = warps * S::bytes(arrays);
   static GroupLaunch st;
   const cudaError_t e = st.prepare(sweep_group_kernel<real, DIM, P1, FM, H>, arrays, grid, block, smem,
-                                   warps * S::bytes(FM >= 1 ? 2 : 1), 0, kGroupKeepKb);
+                                   warps * S::bytes(FM >= 1 ? 2 : 1), 0, a.n_queues > 1 ? kQueueKeepKb : kGroupKeepKb);
   if (e != cudaSuccess) return e;
   sweep_group_kernel<real, DIM, P1, FM, H><<<grid, block, smem, s>>>(a);
   return cudaGetLastError();
