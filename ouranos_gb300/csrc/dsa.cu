@@ -1198,9 +1198,10 @@ int ouranos_rt_dsa_apply(ouranos_rt* rt, const double* v, double* z) {
   const double* dv = nullptr;
   rc = rt_stage_in(rt, v, rt->d_x, 1, &dv);
   if (rc) return rc;
-  DC(rt->d_y.alloc(sizeof(double) * (long)rt->n_mom * rt->n_dofs), "output");
-  if ((rc = rt_dsa_apply(rt, dv, rt->d_y.as<double>()))) return rc;
-  if ((rc = rt_stage_out(rt, rt->d_y.as<double>(), z))) return rc;
+  double* out = nullptr;
+  if ((rc = rt_result_target(rt, dv, z, true, rt->d_y, &out))) return rc;
+  if ((rc = rt_dsa_apply(rt, dv, out))) return rc;
+  if ((rc = rt_stage_out(rt, out, z))) return rc;
   return rt_check_status(rt);
 }
 

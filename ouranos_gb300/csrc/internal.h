@@ -423,6 +423,7 @@ int rt_dsa_apply_batch(ouranos_rt* const* rts, const double* const* v, double* c
                        cudaStream_t stream, int* status, DsaBatchScratch& sc, std::string& err);
 int rt_stage_in(ouranos_rt* rt, const double* v, DevBuf& buf, int n_vec, const double** out);
 int rt_stage_out(ouranos_rt* rt, const double* dv, double* user);
+int rt_result_target(ouranos_rt* rt, const double* in, double* user, bool in_place, DevBuf& buf, double** out);
 }  // namespace ouranos
 
 // cell ranges of the host-vector Apply's overlapped copies
@@ -466,6 +467,7 @@ struct ouranos_rt {
   std::vector<int> dir_class_h;
   ouranos::DevBuf d_queue_tasks, d_queue_first;  // tasks by |Omega| class (SweepArgs::queue_first)
   int n_queues = 1;
+  int* h_status = nullptr;  // page-locked copy of the status word
   std::vector<double> class_abs_omega;  // [n_dir_class][3]
   int n_dir_class = 0;
   std::vector<double> sigma_class_value; // per sigma_t class

@@ -757,9 +757,10 @@ int clear_status(ouranos_rt* rt) {
 }
 
 int finish(ouranos_rt* rt) {
+  // the status word comes back in the stream: one wait, not a second one for the copy
+  CU(cudaMemcpyAsync(rt->h_status, rt->d_ctrl.as<int>() + 1, sizeof(int), cudaMemcpyDeviceToHost, rt->stream), "status");
   CU(cudaStreamSynchronize(rt->stream), "sweep");
-  int st = 0;
-  CU(cudaMemcpy(&st, rt->d_ctrl.as<int>() + 1, sizeof(int), cudaMemcpyDeviceToHost), "status");
+  const int st = *(volatile int*)rt->h_status;
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, rt->ev0, rt->ev1) == cudaSuccess)
     rt->last_ms = ms;
@@ -832,6 +833,28 @@ int stage_out(ouranos_rt* rt, const double* dv, double* user) {
                     rt->n_mom, 0, rt->stream),
      "permute out");
   CU(cudaMemcpyAsync(user, rt->d_tmp.p, bytes, cudaMemcpyDeviceToHost, rt->stream), "copy out");
+  return OURANOS_OK;
+}
+
+// Where a call's result goes: the caller's vector itself where the last kernel may
+// write it (this device's memory in lexicographic numbering, apart from the vector
+// `in` that the kernel reads, or the same with in_place), else `buf`, for stage_out.
+// The copy was a pass over the result of its own: FP32 Apply on 128^3 5159 -> 5106 us;
+// on 32^2 (with the one wait of finish()) 83.9 -> 75.4.
+int result_target(ouranos_rt* rt, const double* in, double* user, bool in_place, DevBuf& buf, double** out) {
+  const size_t len = vec_len(rt);
+  cudaPointerAttributes at;
+  if (rt->cell_order.empty() && (reinterpret_cast<size_t>(user) & 15) == 0 &&
+      ((in_place && in == user) || in + len <= user || user + len <= in)) {
+    if (cudaPointerGetAttributes(&at, user) != cudaSuccess) {
+      cudaGetLastError();
+    } else if (at.type == cudaMemoryTypeDevice && at.device == rt->device) {
+      *out = user;
+      return OURANOS_OK;
+    }
+  }
+  CU(buf.alloc(sizeof(double) * len), "result");
+  *out = buf.as<double>();
   return OURANOS_OK;
 }
 
@@ -1112,6 +1135,9 @@ int rt_stage_in(ouranos_rt* rt, const double* v, DevBuf& buf, int n_vec, const d
   return stage_in(rt, v, buf, n_vec, out);
 }
 int rt_stage_out(ouranos_rt* rt, const double* dv, double* user) { return stage_out(rt, dv, user); }
+int rt_result_target(ouranos_rt* rt, const double* in, double* user, bool in_place, DevBuf& buf, double** out) {
+  return result_target(rt, in, user, in_place, buf, out);
+}
 }  // namespace ouranos
 
 // ===================================================================== C-ABI
@@ -1213,7 +1239,8 @@ int ouranos_rt_create(const ouranos_problem_desc* D, int device, ouranos_rt** ou
   // legacy default stream (and before work issued there later), so device
   // vectors a caller has just written on that stream are read complete.
   if (cudaStreamCreateWithFlags(&rt->own_stream, cudaStreamDefault) != cudaSuccess ||
-      cudaEventCreate(&rt->ev0) != cudaSuccess || cudaEventCreate(&rt->ev1) != cudaSuccess)
+      cudaEventCreate(&rt->ev0) != cudaSuccess || cudaEventCreate(&rt->ev1) != cudaSuccess ||
+      cudaMallocHost((void**)&rt->h_status, sizeof(int)) != cudaSuccess)
     return fail(cuda_fail(rt, cudaGetLastError(), "stream"));
   rt->stream = rt->own_stream;
   // the allocation-free Apply's scratch array is placed on the device here,
@@ -1312,6 +1339,7 @@ int ouranos_rt_destroy(ouranos_rt* rt) {
     cudaSetDevice(rt->device);
     cudaStreamSynchronize(rt->stream);
   }
+  if (rt->h_status) cudaFreeHost(rt->h_status);
   if (rt->ev0) cudaEventDestroy(rt->ev0);
   if (rt->ev1) cudaEventDestroy(rt->ev1);
   for (cudaEvent_t e : rt->ev_chunk)
@@ -1405,9 +1433,10 @@ int ouranos_rt_sweep(ouranos_rt* rt, double* flux, const double* group_flux) {
   OK_OR_RETURN(sweep_into_phi(rt, group_flux != nullptr));
   const double* dflux = nullptr;
   OK_OR_RETURN(stage_in(rt, flux, rt->d_x, 1, &dflux));
-  CU(rt->d_y.alloc(sizeof(double) * vec_len(rt)), "flux");
-  OK_OR_RETURN(phi_combine(rt, dflux, rt->d_y.as<double>(), 1.0, 1.0));  // flux + phi
-  OK_OR_RETURN(stage_out(rt, rt->d_y.as<double>(), flux));
+  double* out = nullptr;
+  OK_OR_RETURN(result_target(rt, dflux, flux, true, rt->d_y, &out));
+  OK_OR_RETURN(phi_combine(rt, dflux, out, 1.0, 1.0));  // flux + phi
+  OK_OR_RETURN(stage_out(rt, out, flux));
   return finish(rt);
 }
 
@@ -1424,9 +1453,10 @@ int ouranos_rt_apply(ouranos_rt* rt, const double* x, double* y) {
   }
   const double* dx = nullptr;
   OK_OR_RETURN(stage_in(rt, x, rt->d_x, 1, &dx));
-  CU(rt->d_y.alloc(sizeof(double) * vec_len(rt)), "apply");
-  OK_OR_RETURN(rt_apply_device(rt, dx, rt->d_y.as<double>()));
-  OK_OR_RETURN(stage_out(rt, rt->d_y.as<double>(), y));
+  double* out = nullptr;
+  OK_OR_RETURN(result_target(rt, dx, y, false, rt->d_y, &out));
+  OK_OR_RETURN(rt_apply_device(rt, dx, out));
+  OK_OR_RETURN(stage_out(rt, out, y));
   return finish(rt);
 }
 
@@ -1440,9 +1470,10 @@ int ouranos_rt_sweep_rhs(ouranos_rt* rt, const double* group_flux, double* rhs) 
   OK_OR_RETURN(sweep_into_phi(rt, true));
   const double* drhs = nullptr;
   OK_OR_RETURN(stage_in(rt, rhs, rt->d_x, 1, &drhs));
-  CU(rt->d_y.alloc(sizeof(double) * vec_len(rt)), "rhs");
-  OK_OR_RETURN(phi_combine(rt, drhs, rt->d_y.as<double>(), 1.0, 1.0));
-  OK_OR_RETURN(stage_out(rt, rt->d_y.as<double>(), rhs));
+  double* out = nullptr;
+  OK_OR_RETURN(result_target(rt, drhs, rhs, true, rt->d_y, &out));
+  OK_OR_RETURN(phi_combine(rt, drhs, out, 1.0, 1.0));
+  OK_OR_RETURN(stage_out(rt, out, rhs));
   return finish(rt);
 }
 
