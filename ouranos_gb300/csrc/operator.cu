@@ -303,6 +303,9 @@ size_t edge_bytes(const ouranos_rt* rt, int wx, int wy) {
 // batch counts as a large problem: the batch's launch is full anyway, and fewer
 // forms are fewer launches.  Two lanes to a cell have the nominal tiling's tiles:
 // the last resort of the orders without a per-lane kernel.
+bool fp64_cell_solves(const ouranos_rt* rt) {
+  return rt->fp64_contract == OURANOS_FP64_NATIVE || rt->fp64_contract == OURANOS_FP64_DF64;
+}
 int default_tiling(ouranos_rt* rt) {
   rt->kd = 1;
   int wx0 = 0, wy0 = 0, lpc0 = 0;
@@ -325,6 +328,14 @@ int default_tiling(ouranos_rt* rt) {
     }
   }
   if (rt->n_mom == 2 && rt->n * 3 <= 32) lanes.clear();  // two fused moments: the per-lane form
+  // FP64 cell solves: bound by the FP64 pipe, which wants few idle lanes and tiles
+  // spread evenly (sweep kernel, ms, nominal / default form above: 2-D Q2 256^2 LS S16
+  // 2.52 / 3.44, 3-D Q1 48^3 LS S8 2.74 / 2.87, 3-D Q3 12^3 LS S4 0.80 / 0.91; but 2-D Q2
+  // 64^2 0.36 / 0.26, 2-D Q1 256^2 1.01 / 0.98, and no per-lane kernel for 2-D Q3, Q4
+  // and 3-D Q2).  A batch keeps one form for both of its precisions.
+  if (fp64_cell_solves(rt) && !rt->in_batch &&
+      (rt->dim == 2 ? rt->p1 == 6 || (rt->p1 == 3 && !lanes.empty() && lanes[0] == 1) : rt->p1 == 2 || rt->p1 >= 4))
+    lanes.clear();
   // one lane per cell counts dofs in an int (also of the planes the tile's skew
   // walks in from)
   const long plane = rt->n_cells / rt->nx[rt->dim - 1];
@@ -1379,7 +1390,21 @@ int ouranos_rt_set_fp64_contractions(ouranos_rt* rt, int mode) {
     rt->err = "tensor-core FP64 contractions take at most 192 directions and 16 moments";
     return OURANOS_ERR_UNSUPPORTED;
   }
+  const bool before = fp64_cell_solves(rt);
   rt->fp64_contract = mode;
+  // the default form may be another one for FP64 cell solves
+  if (fp64_cell_solves(rt) != before && rt->tiling[0] == 0 && !rt->in_batch) {
+    cudaSetDevice(rt->device);
+    const int wx = rt->wx, wy = rt->wy, lpc = rt->lpc;
+    const bool grouped = rt->grouped;
+    OK_OR_RETURN(default_tiling(rt));
+    if (wx != rt->wx || wy != rt->wy || lpc != rt->lpc || grouped != rt->grouped) {
+      CU(cudaStreamSynchronize(rt->stream), "tiling");
+      OK_OR_RETURN(build_schedule(rt));
+      OK_OR_RETURN(setup_group(rt));
+      CU(cudaStreamSynchronize(rt->stream), "tiling");
+    }
+  }
   return OURANOS_OK;
 }
 

@@ -128,3 +128,30 @@ def test_wait_timeout_reports_error_and_recovers(dim, order, n):
         rt.debug_wait_bias(0)
         rt.set_wait_limit(2e9)
         assert np.array_equal(rt.apply(x), ref)
+
+
+@pytest.mark.parametrize("dim,order,n,sn", [(2, 2, (34, 6), 16), (3, 1, (5, 9, 7), 4), (3, 3, (3, 2, 3), 4),
+                                            (2, 1, (33, 5), 4)])
+def test_form_follows_the_arithmetic(dim, order, n, sn):
+    """FP64 cell solves take another default form for some orders: switching back and
+    forth, with either precision, gives what a fresh handle in that mode gives."""
+    import ouranos_gb300 as og
+    prob = _problem(og, dim, order, n, sn, 1)
+    x = np.random.default_rng(9).standard_normal(prob.vector_length)
+    fresh = {}
+    for mode in ("df64_sweep", "native", "df64"):
+        with og.RadiativeTransfer(prob) as rt:
+            rt.set_fp64_contractions(mode)
+            rt.set_dsa(2) if order <= 2 else None
+            fresh[mode] = rt.apply(x), rt.rhs()
+    with og.RadiativeTransfer(prob, precision="fp32") as rt:
+        y32 = rt.apply(x)
+    with og.RadiativeTransfer(prob) as rt:
+        for mode in ("native", "df64_sweep", "df64", "native", "df64_sweep"):
+            rt.set_fp64_contractions(mode)
+            for _ in range(2):
+                assert np.array_equal(rt.apply(x), fresh[mode][0])
+            assert np.array_equal(rt.rhs(), fresh[mode][1])
+            rt.set_precision("fp32")
+            assert np.array_equal(rt.apply(x), y32)
+            rt.set_precision("fp64")
