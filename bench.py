@@ -72,13 +72,13 @@ def workload_config(cells, directions, moments, dofs_per_cell, world):
 
 # DRAM traffic of one sweep launch on the default workload
 # (dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of the
-# default tiling, 16 x 1 cells with two lanes per cell, in the default FP64
-# arithmetic and in FP32), keyed by a digest of the sweep kernel's sources at
+# default form, one lane per cell in tiles of 32, whose nominal tiling is
+# 16 x 1, in the default FP64 arithmetic), keyed by a digest of its sources at
 # the time of the capture: after any change to those sources the figure no
 # longer describes the kernel and the line reports traffic as null.
 PROFILED_TILING = (16, 1, 1)
-SWEEP_SOURCES = ("sweep.cuh", "sweep_df64.cu", "sweep_f32.cu", "df64.cuh")
-SWEEP_TRAFFIC = {"digest": "67f909790da3fada", "bytes": {"fp64": 701016576 + 663608064}}
+SWEEP_SOURCES = ("sweep_lane.cuh", "sweep_lane_df64.cu", "sweep_group.cuh", "sweep.cuh", "pack2.cuh")
+SWEEP_TRAFFIC = {"digest": "787012ed0bb8d950", "bytes": {"fp64": 696841728 + 644420864}}
 
 
 def sweep_source_digest():
