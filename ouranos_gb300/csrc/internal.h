@@ -110,7 +110,9 @@ struct SweepArgs {
   const real* src;             // [n_mom][n_dofs] source moments T (moment-fused form)
   const real* iso;             // [n_dofs] isotropic fixed source or NULL (moment-fused form)
   const real* q;               // [n_dir][n_dofs] per-direction source (expanded form)
-  const real* bnd;             // [n_dir][3] boundary inflow per axis or NULL
+  const real* bnd;             // [n_dir][3] boundary inflow per axis, zeros where nothing flows in (no
+                               // loads that only some calls make: every build of the sweep
+                               // that ended in a memory fault did so in a call that made them)
   real* psi;                   // [n_dir][n_dofs] angular flux out
   // edge buffers of tagged 64-bit words (1 per FP32 value, 2 per FP64 value)
   unsigned long long* edge_x;  // [n_dir][tiles][n_sweep][wy][fd][words]
@@ -487,6 +489,7 @@ struct ouranos_rt {
   ouranos::DevBuf d_dir_class, d_abs64, d_abs32, d_m2d64, d_m2d32, d_d2m64, d_d2m32;
   ouranos::DevBuf d_ainv64, d_ainv32, d_face64, d_face32, d_bnd64, d_bnd32;
   ouranos::DevBuf d_absdf, d_m2ddf, d_ainvdf, d_facedf, d_bnddf;  // double-float sweep tables
+  ouranos::DevBuf d_no_inflow;  // [n_dir][3] zeros of any precision
   ouranos::DevBuf d_tasks, d_group_dirs, d_group_flip, d_progress, d_ctrl;
   ouranos::DevBuf d_edge_x, d_edge_y;
   // device: vectors

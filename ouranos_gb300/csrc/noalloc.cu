@@ -231,7 +231,7 @@ int apply_noalloc(ouranos_rt* rt, unsigned char* base, const Layout& L, bool exp
   a.src = T;
   a.iso = nullptr;
   a.q = q;
-  a.bnd = nullptr;
+  a.bnd = rt->d_no_inflow.as<real>();
   a.psi = psi;
   a.edge_x = reinterpret_cast<unsigned long long*>(base + L.edge_x);
   a.edge_y = reinterpret_cast<unsigned long long*>(base + L.edge_y);

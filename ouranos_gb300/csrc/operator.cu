@@ -629,7 +629,7 @@ int sweep_prepare(ouranos_rt* rt, const real* src, const real* iso, const real* 
   a.src = src;
   a.iso = iso;
   a.q = nullptr;
-  a.bnd = bnd;
+  a.bnd = bnd ? bnd : rt->d_no_inflow.as<real>();
   CU(rt->d_psi.alloc(sizeof(real) * len_dir), "angular flux");
   a.psi = rt->d_psi.as<real>();
   a.edge_x = rt->d_edge_x.as<unsigned long long>();
@@ -1303,7 +1303,8 @@ int ouranos_rt_create(const ouranos_problem_desc* D, int device, ouranos_rt** ou
       (rc = upload(rt, rt->d_cell_mass, rt->fe.mass, "mass")) ||
       (rc = upload(rt, rt->d_rowsum_mass, rowsum, "mass")) ||
       (rc = upload(rt, rt->d_material, rt->material_id, "materials")) ||
-      (rc = upload(rt, rt->d_source_id, sid, "source ids")))
+      (rc = upload(rt, rt->d_source_id, sid, "source ids")) ||
+      (rc = upload(rt, rt->d_no_inflow, std::vector<double>((size_t)rt->n_dir * 3, 0.0), "boundary")))
     return fail(rc);
   if (!rt->cell_order.empty() && (rc = upload(rt, rt->d_cell_order, rt->cell_order, "cell order")))
     return fail(rc);

@@ -154,6 +154,7 @@ struct Arith {
   static __device__ __forceinline__ real ldg(const real* p) { return __ldg(p); }
   static __device__ __forceinline__ real shfl_up(real v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
   static __device__ __forceinline__ real shfl_xor(real v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
+  static __device__ __forceinline__ real shfl(real v, int l) { return __shfl_sync(0xffffffffu, v, l); }
 };
 template <>
 struct Arith<df64> {
@@ -175,6 +176,9 @@ struct Arith<df64> {
   }
   static __device__ __forceinline__ df64 shfl_xor(df64 v, int m) {
     return df64(__shfl_xor_sync(0xffffffffu, v.hi, m), __shfl_xor_sync(0xffffffffu, v.lo, m));
+  }
+  static __device__ __forceinline__ df64 shfl(df64 v, int l) {
+    return df64(__shfl_sync(0xffffffffu, v.hi, l), __shfl_sync(0xffffffffu, v.lo, l));
   }
 };
 
@@ -475,12 +479,9 @@ __device__ __forceinline__ void sweep_task(const SweepArgs<real> a, const int ta
     const real wX = a.abs_omega[dd * 3 + 0];
     const real wY = DIM == 3 ? a.abs_omega[dd * 3 + 1] : real(0);
     const real wS = a.abs_omega[dd * 3 + AS];
-    real bX = 0, bY = 0, bS = 0;
-    if (a.bnd) {
-      bX = a.bnd[dd * 3 + 0];
-      if (DIM == 3) bY = a.bnd[dd * 3 + 1];
-      bS = a.bnd[dd * 3 + AS];
-    }
+    const real bX = a.bnd[dd * 3 + 0];
+    const real bY = DIM == 3 ? a.bnd[dd * 3 + 1] : real(0);
+    const real bS = a.bnd[dd * 3 + AS];
     real w0 = 0, w1 = 0;  // M2D row (moment-fused form)
     if (FM >= 1) w0 = a.m2d[(size_t)dd * a.n_mom + 0];
     if (FM >= 2) w1 = a.m2d[(size_t)dd * a.n_mom + 1];

@@ -166,12 +166,12 @@ __device__ __forceinline__ void sweep_group_task(const SweepArgs<real>& a, const
   const real wX = a.abs_omega[d * 3 + 0];
   const real wY = DIM == 3 ? a.abs_omega[d * 3 + 1] : real(0);
   const real wS = a.abs_omega[d * 3 + AS];
-  real bX = 0, bY = 0, bS = 0, w0 = 0;
-  if (a.bnd) {
-    bX = a.bnd[d * 3 + 0];
-    if (DIM == 3) bY = a.bnd[d * 3 + 1];
-    bS = a.bnd[d * 3 + AS];
-  }
+  // Inflow: a.bnd is a table of zeros where there is none, so that every call takes the
+  // same path, and the values pass through a shuffle, which the whole warp waits for
+  const real bX = A::shfl(a.bnd[d * 3 + 0], 0);
+  const real bY = DIM == 3 ? A::shfl(a.bnd[d * 3 + 1], 0) : real(0);
+  const real bS = A::shfl(a.bnd[d * 3 + AS], 0);
+  real w0 = 0;
   if (FM >= 1) w0 = a.m2d[(size_t)d * a.n_mom];
   // physical position of canonical dof i: base + c0 st0 + c1 st1 + c2 st2
   int base = 0, st0 = 1, st1 = P1, st2 = P1 * P1;
@@ -230,11 +230,14 @@ __device__ __forceinline__ void sweep_group_task(const SweepArgs<real>& a, const
 
   __syncwarp();  // the slot's last task has been read to its end
   // upwind values at the start: the boundary's, until a neighbour's or an edge's
+  // (every lane writes its row's and its column's ghost cell, the lanes of one alike; the
+  // barrier orders the first step's edge words after them)
   for (int i = h; i < N; i += H) {
     put(s_x, i, bS);
-    if (lx == 0) put(s_gx, i, bX);
-    if (DIM == 3 && ly == 0) put(s_gy, i, bY);
+    put(s_gx, i, bX);
+    if (DIM == 3) put(s_gy, i, bY);
   }
+  __syncwarp();
 #pragma unroll
   for (int j = 0; j < S::PF; ++j) issue(j, j - lx - ly, cell + j * cstep);
 

@@ -137,12 +137,12 @@ __device__ __forceinline__ void sweep_lane_task(const SweepArgs<real>& a, const 
   const real wX = a.abs_omega[d * 3 + 0];
   const real wY = DIM == 3 ? a.abs_omega[d * 3 + 1] : real(0);
   const real wS = a.abs_omega[d * 3 + AS];
-  real bX = 0, bY = 0, bS = 0, w0 = 0;
-  if (a.bnd) {
-    bX = a.bnd[d * 3 + 0];
-    if (DIM == 3) bY = a.bnd[d * 3 + 1];
-    bS = a.bnd[d * 3 + AS];
-  }
+  // Inflow: a.bnd is a table of zeros where there is none, so that every call takes the
+  // same path, and the values pass through a shuffle, which the whole warp waits for
+  const real bX = A::shfl(a.bnd[d * 3 + 0], 0);
+  const real bY = DIM == 3 ? A::shfl(a.bnd[d * 3 + 1], 0) : real(0);
+  const real bS = A::shfl(a.bnd[d * 3 + AS], 0);
+  real w0 = 0;
   if (FM >= 1) w0 = a.m2d[(size_t)d * a.n_mom];
   // physical position of canonical dof i: base + c0 st0 + c1 st1 + c2 st2
   int base = 0, st0 = 1, st1 = P1, st2 = P1 * P1;
@@ -225,10 +225,14 @@ __device__ __forceinline__ void sweep_lane_task(const SweepArgs<real>& a, const 
   };
 
   __syncwarp();  // the slot's last task has been read to its end
-  if (lx == 0)
-    for (int t = 0; t < FD; ++t) *reinterpret_cast<real*>(sm + S::o_ex + ly * S::EB + t * SZ) = bX;
-  if (DIM == 3 && ly == 0)
-    for (int t = 0; t < FD; ++t) *reinterpret_cast<real*>(sm + S::o_ey + lx * S::EB + t * SZ) = bY;
+  // The inflow, until an edge brings a neighbour's values: every lane writes it to its
+  // row's and its column's slot (the same value from all lanes of one).  The edge words
+  // of the first step are written by other lanes than these: the barrier orders the two.
+  for (int t = 0; t < FD; ++t) {
+    *reinterpret_cast<real*>(sm + S::o_ex + ly * S::EB + t * SZ) = bX;
+    if (DIM == 3) *reinterpret_cast<real*>(sm + S::o_ey + lx * S::EB + t * SZ) = bY;
+  }
+  __syncwarp();
   class_word(0);
   class_word(1);
 #pragma unroll

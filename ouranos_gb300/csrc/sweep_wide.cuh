@@ -79,12 +79,9 @@ __device__ __forceinline__ void sweep_wide_task(const SweepArgs<real>& a, const 
   const real wX = a.abs_omega[d * 3 + 0];
   const real wY = DIM == 3 ? a.abs_omega[d * 3 + 1] : real(0);
   const real wS = a.abs_omega[d * 3 + AS];
-  real bX = 0, bY = 0, bS = 0;
-  if (a.bnd) {
-    bX = a.bnd[d * 3 + 0];
-    if (DIM == 3) bY = a.bnd[d * 3 + 1];
-    bS = a.bnd[d * 3 + AS];
-  }
+  const real bX = a.bnd[d * 3 + 0];
+  const real bY = DIM == 3 ? a.bnd[d * 3 + 1] : real(0);
+  const real bS = a.bnd[d * 3 + AS];
   const int dcls = a.dir_class[d];
   // mirrored local dof offsets: phys(i') = base + c0*s0 + c1*s1 + c2*s2
   int base = 0, st0 = 1, st1 = P1, st2 = P1 * P1;
