@@ -87,6 +87,10 @@ inline bool per_lane_order(int dim, int p1) { return dim == 2 ? p1 <= 5 : p1 <= 
 inline bool per_lane_kernel(int dim, int p1) { return dim == 2 ? p1 <= 3 : p1 == 2; }
 
 // ---------------------------------------------------------- sweep kernels
+// The default forms stream their sources in aligned 16-byte pieces, the last of which
+// may reach past the last value (27 FP32 values at the start of a piece take seven,
+// eight are read: 20 bytes): every source buffer is this much longer.
+constexpr size_t kSrcSlack = 32;
 // Arguments of one sweep launch (see sweep.cuh for the algorithm).
 template <typename real>
 struct SweepArgs {

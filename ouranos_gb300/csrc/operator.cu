@@ -16,10 +16,6 @@ using namespace ouranos;
 
 namespace {
 
-// the sweep streams its sources in aligned 16-byte pieces, the last of which may
-// reach past the last value: every source buffer is this much longer
-constexpr size_t kSrcSlack = 16;
-
 #define OK_OR_RETURN(expr)                 \
   do {                                     \
     int _rc = (expr);                      \

@@ -75,6 +75,7 @@ struct GroupSlot {
   static constexpr int CELLB = N * SZ;
   static constexpr int GR = (CELLB & -CELLB) < 16 ? (CELLB & -CELLB) : 16;
   static constexpr int CH = (CELLB + 16 - GR + 15) / 16;
+  static_assert(16 * CH - CELLB <= (int)kSrcSlack, "the sources' buffers hold the last piece");
   // strides of odd multiples of 16 bytes: the cells of a warp start on different banks
   static constexpr int SRC = 16 * (CH | 1);
   static constexpr int VEC = 16 * (((N * SZ + 15) / 16) | 1);

@@ -35,6 +35,7 @@ struct LaneSlot {
   static constexpr int CELLB = N * SZ;
   static constexpr int GR = (CELLB & -CELLB) < 16 ? (CELLB & -CELLB) : 16;
   static constexpr int CH = (CELLB + 16 - GR + 15) / 16;  // aligned 16-byte pieces that cover a cell's source
+  static_assert(16 * CH - CELLB <= (int)kSrcSlack, "the sources' buffers hold the last piece");
   static constexpr int SRC = 16 * (CH | 1);               // (odd multiples of 16 bytes: different banks)
   // psi's slot: Q1 cells padded likewise; 9 values at their own stride, which meets
   // every bank once and makes the slot one array of the tile's values
