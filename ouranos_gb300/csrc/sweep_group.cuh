@@ -20,7 +20,6 @@
 // forms, whatever H is, so all forms give the same bits.
 #pragma once
 
-#include <mutex>
 #include <type_traits>
 
 #include "pack2.cuh"
@@ -663,34 +662,6 @@ __global__ void __launch_bounds__(128) sweep_group_kernel(const __grid_constant_
   }
 }
 
-// Launch settings of one kernel, found once per process: the opt-in to its
-// shared memory, its resident blocks, and the last carveout asked for.
-struct GroupLaunch {
-  std::mutex mu;
-  int max_per_sm[2] = {0, 0}, carve = -2;  // (by the number of source arrays)
-  template <typename K>
-  cudaError_t prepare(K kernel, int arrays, int grid, int block, size_t smem, size_t smem_max, size_t smem_static,
-                      int keep_kb) {
-    std::lock_guard<std::mutex> lock(mu);
-    int& per_sm = max_per_sm[arrays - 1];
-    if (!per_sm) {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
-      if (e != cudaSuccess) return e;
-      int n = 0;
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block, smem);
-      if (e != cudaSuccess) return e;
-      per_sm = n > 0 ? n : 1;
-    }
-    const int pct = carveout_percent(grid, smem + smem_static, per_sm, keep_kb);
-    if (pct >= 0 && pct != carve) {
-      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
-      if (e != cudaSuccess) return e;
-      carve = pct;
-    }
-    return cudaSuccess;
-  }
-};
-
 // What a batched launch of a form needs: every problem's arguments, the ticket
 // map, and whether the problems bring a fixed source
 template <typename real>
@@ -732,8 +703,8 @@ cudaError_t launch_group_fm(const SweepArgs<real>& a, int grid, int block, cudaS
   using S = GroupSlot<real, DIM, P1, H>;
   const int arrays = FM >= 1 && a.iso ? 2 : 1;
   const size_t warps = block / 32, smem = warps * S::bytes(arrays);
-  static GroupLaunch st;
-  const cudaError_t e = st.prepare(sweep_group_kernel<real, DIM, P1, FM, H>, arrays, grid, block, smem,
+  static SweepLaunch st;
+  const cudaError_t e = st.prepare((const void*)sweep_group_kernel<real, DIM, P1, FM, H>, arrays, grid, block, smem,
                                    warps * S::bytes(FM >= 1 ? 2 : 1), 0, a.n_queues > 1 ? kQueueKeepKb : kGroupKeepKb);
   if (e != cudaSuccess) return e;
   sweep_group_kernel<real, DIM, P1, FM, H><<<grid, block, smem, s>>>(a);
@@ -744,8 +715,8 @@ cudaError_t launch_group_batch_fm(const BatchLaunch<real>& b, cudaStream_t s) {
   using S = GroupSlot<real, DIM, P1, H>;
   const int arrays = FM >= 1 && b.sources ? 2 : 1;
   const size_t warps = b.block / 32, smem = warps * S::bytes(arrays);
-  static GroupLaunch st;
-  const cudaError_t e = st.prepare(sweep_group_batch_kernel<real, DIM, P1, FM, H>, arrays, b.grid, b.block, smem,
+  static SweepLaunch st;
+  const cudaError_t e = st.prepare((const void*)sweep_group_batch_kernel<real, DIM, P1, FM, H>, arrays, b.grid, b.block, smem,
                                    warps * S::bytes(FM >= 1 ? 2 : 1), 4 * sizeof(SweepArgs<real>), kGroupKeepKb);
   if (e != cudaSuccess) return e;
   sweep_group_batch_kernel<real, DIM, P1, FM, H>

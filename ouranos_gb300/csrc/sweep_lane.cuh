@@ -674,8 +674,8 @@ cudaError_t launch_lane_fm(const SweepArgs<real>& a, int grid, int block, cudaSt
   using S = LaneSlot<real, DIM, P1>;
   const int arrays = FM >= 1 && a.iso ? 2 : 1;
   const size_t warps = block / 32, smem = warps * S::bytes(arrays);
-  static GroupLaunch st;
-  const cudaError_t e = st.prepare(sweep_lane_kernel<real, DIM, P1, FM>, arrays, grid, block, smem,
+  static SweepLaunch st;
+  const cudaError_t e = st.prepare((const void*)sweep_lane_kernel<real, DIM, P1, FM>, arrays, grid, block, smem,
                                    warps * S::bytes(FM >= 1 ? 2 : 1), 0, kGroupKeepKb);
   if (e != cudaSuccess) return e;
   sweep_lane_kernel<real, DIM, P1, FM><<<grid, block, smem, s>>>(a);
@@ -686,8 +686,8 @@ cudaError_t launch_lane_batch_fm(const BatchLaunch<real>& b, cudaStream_t s) {
   using S = LaneSlot<real, DIM, P1>;
   const int arrays = FM >= 1 && b.sources ? 2 : 1;
   const size_t warps = b.block / 32, smem = warps * S::bytes(arrays);
-  static GroupLaunch st;
-  const cudaError_t e = st.prepare(sweep_lane_batch_kernel<real, DIM, P1, FM>, arrays, b.grid, b.block, smem,
+  static SweepLaunch st;
+  const cudaError_t e = st.prepare((const void*)sweep_lane_batch_kernel<real, DIM, P1, FM>, arrays, b.grid, b.block, smem,
                                    warps * S::bytes(FM >= 1 ? 2 : 1), 4 * sizeof(SweepArgs<real>), kGroupKeepKb);
   if (e != cudaSuccess) return e;
   sweep_lane_batch_kernel<real, DIM, P1, FM>
