@@ -40,6 +40,7 @@
 #include <cstdio>
 #include <vector>
 
+#include "fsum.cuh"
 #include "internal.h"
 
 using namespace ouranos;
@@ -214,15 +215,6 @@ struct Meeting {
   unsigned passed = 0;
 };
 
-// (t, e) += (o, oe): a float pair, Knuth's two-sum of the leading parts, some 48 bits
-__device__ __forceinline__ void pair_add(float& t, float& e, float o, float oe) {
-  const float s = __fadd_rn(t, o);
-  const float bb = __fsub_rn(s, t);
-  const float err = __fadd_rn(__fsub_rn(t, __fsub_rn(s, bb)), __fsub_rn(o, bb));
-  t = s;
-  e = __fadd_rn(__fadd_rn(e, oe), err);
-}
-
 __device__ __forceinline__ double warp_sum(double u) {
   for (int o = 16; o; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
   return u;
@@ -230,34 +222,29 @@ __device__ __forceinline__ double warp_sum(double u) {
 
 // sums[i] = the problem's sum of t[i] (its nb blocks, this one number lb, with a
 // partial each in part[i]); thread 0 turns the sums into one number, finish(sums),
-// which every thread returns in `result`.  A block adds its threads' FP32 values as
-// float pairs (exact sums with their errors kept), the block partials are FP64 and
-// added in block order by every block alike: deterministic, the same everywhere.
-// (GB300 adds two FP64 lanes a clock: the 32 warps' FP64 shuffle trees cost 3400
-// clocks a sum, the pairs some 600; and one thread divides, as 1024 FP64
-// divisions took 5000 clocks.)  A warp whose pair sum leaves the FP32 range adds
-// in FP64.
+// which every thread returns in `result`.  A warp adds its threads' FP32 values in
+// fixed point (fsum.cuh), the rest is FP64: the warps' totals by one warp's shuffles,
+// the block partials in block order by every block alike: deterministic, the same
+// everywhere, and no less than the FP64 trees of all 32 warps gave.  (GB300 adds two
+// FP64 lanes a clock: those trees cost 3400 clocks a sum; and one thread divides, as
+// 1024 FP64 divisions took 5000 clocks.  20 steps on 64^3: 257 us; with the warps' sums
+// as float pairs, some 48 bits only, 251.)  A warp with an infinite value or a NaN adds in FP64.
 template <int NV, typename F>
 __device__ __forceinline__ bool meet(Meeting& m, const float (&t)[NV], double* const (&part)[NV], int lb, int nb,
                                      float& result, F finish) {
-  __shared__ float wsum[NV][2][kCgThreads / 32];
-  __shared__ double wide[NV][kCgThreads / 32];  // of warps whose pair sum left the FP32 range
+  __shared__ int64_t wsum[NV][kCgThreads / 32];
+  __shared__ int wexp[NV][kCgThreads / 32];
   __shared__ float answer;
   __shared__ int ok;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    float s = t[i], e = 0.f;
-#pragma unroll
-    for (int o = 16; o; o >>= 1)
-      pair_add(s, e, __shfl_xor_sync(0xffffffffu, s, o), __shfl_xor_sync(0xffffffffu, e, o));
+    int emax;
+    int64_t total = warp_fixed_sum(t[i], emax);
+    if (emax == 255) total = __double_as_longlong(warp_sum((double)t[i]));  // (the same in all lanes)
     if (lane == 0) {
-      wsum[i][0][warp] = s;
-      wsum[i][1][warp] = e;
-    }
-    if (!isfinite(s)) {  // (the same in all lanes)
-      const double d = warp_sum((double)t[i]);
-      if (lane == 0) wide[i][warp] = d;
+      wsum[i][warp] = total;
+      wexp[i][warp] = emax;
     }
   }
   __syncthreads();
@@ -266,13 +253,9 @@ __device__ __forceinline__ bool meet(Meeting& m, const float (&t)[NV], double* c
     double mine[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      const float s0 = wsum[i][0][lane], e0 = wsum[i][1][lane];
-      float s = s0, e = e0;
-#pragma unroll
-      for (int o = 16; o; o >>= 1)
-        pair_add(s, e, __shfl_xor_sync(0xffffffffu, s, o), __shfl_xor_sync(0xffffffffu, e, o));
-      mine[i] = isfinite(s) ? (double)s + (double)e
-                            : warp_sum(isfinite(s0) ? (double)s0 + (double)e0 : wide[i][lane]);
+      const int64_t total = wsum[i][lane];
+      const int emax = wexp[i][lane];
+      mine[i] = warp_sum(emax == 255 ? __longlong_as_double(total) : fixed_value(total, emax));
     }
     int fine = 1;
     if (lane == 0) {
