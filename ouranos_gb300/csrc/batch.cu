@@ -36,7 +36,10 @@ using namespace ouranos;
 
 namespace {
 
-constexpr int kMaxClasses = 16;
+// Classes of one batch: fused moments 0, 1, 2 for 2-D Q1, Q2 and 3-D Q1 (2-D Q3: 0, 1;
+// others 0) by the forms an order runs in, the default's 1, 2 or 8 lanes and the
+// tilings the autotuner may pick (1 or 2 lanes): 5 + 8 + 4 + 2 + 5 + 2 = 26.
+constexpr int kMaxClasses = 32;
 constexpr int kStatus = kMaxClasses;      // d_ctrl[kStatus]: sticky timeout flag
 constexpr int kEpoch = kMaxClasses + 1;   // d_ctrl[kEpoch]: edge-word epoch
 constexpr size_t kMaxGraphs = 64;         // captured Apply graphs kept per batch
