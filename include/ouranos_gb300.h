@@ -203,9 +203,20 @@ int ouranos_rt_last_sweep_ms(const ouranos_rt* rt, double* ms, int* kernels);
  * lanes per cell and 16 cells where allowed: 2-D 16 x 1, 3-D 4 x 4; one warp per
  * cell for 2-D Q5 and 3-D Q3..Q5).  2-D Q3 and Q4 and 3-D Q2 accept the same
  * tilings but choose their lanes themselves under all of them but 1 x 1 x 1.
- * Every tiling gives the same bits. */
+ * The nominal tiling itself means the default too, so a tiling that was read and
+ * set again keeps the form.  Every tiling gives the same bits. */
 int ouranos_rt_set_tiling(ouranos_rt* rt, int cells_x, int cells_y, int dirs_per_warp);
 int ouranos_rt_get_tiling(const ouranos_rt* rt, int* cells_x, int* cells_y, int* dirs_per_warp);
+/* The form the handle's sweeps run in: cells and directions of a warp's tile, lanes
+ * that share a cell, and whether it is one of the default forms (1) or a kernel of
+ * the explicit tilings (0).  The default depends on the DG order, the problem's size,
+ * the FP64 arithmetic and, where the smaller tiles' buffers would be a good part of
+ * it, on the memory free on the device when the handle is created. */
+int ouranos_rt_get_form(const ouranos_rt* rt, int* cells_x, int* cells_y, int* dirs_per_warp, int* lanes_per_cell,
+                        int* default_form);
+/* Test hook: 1 makes the default the kernel of the nominal tiling where that has one
+ * of its own (not 2-D Q3, Q4 and 3-D Q2), 0 the library's choice again. */
+int ouranos_rt_debug_nominal_form(ouranos_rt* rt, int on);
 /* Spin limit of the in-kernel dependency waits, in nanoseconds (default 2 s).
  * A wait that runs out sets an error status, every warp leaves, and the call
  * returns OURANOS_ERR_TIMEOUT with the context still usable. */

@@ -36,6 +36,7 @@ EXPORTS = [
     "ouranos_rt_sweep_rhs", "ouranos_rt_task_levels", "ouranos_wavefront_levels",
     "ouranos_rt_set_stream", "ouranos_rt_last_error",
     "ouranos_rt_last_sweep_ms", "ouranos_rt_set_tiling", "ouranos_rt_get_tiling",
+    "ouranos_rt_get_form", "ouranos_rt_debug_nominal_form",
     "ouranos_rt_set_wait_limit", "ouranos_rt_debug_wait_bias", "ouranos_solve",
     "ouranos_rt_apply_noalloc",
     "ouranos_cnn_create", "ouranos_cnn_destroy", "ouranos_cnn_n_params", "ouranos_cnn_get_params",
@@ -118,6 +119,8 @@ def lib():
         "ouranos_rt_last_sweep_ms": [vp, C.POINTER(d), C.POINTER(i)],
         "ouranos_rt_set_tiling": [vp, i, i, i],
         "ouranos_rt_get_tiling": [vp, C.POINTER(i), C.POINTER(i), C.POINTER(i)],
+        "ouranos_rt_get_form": [vp] + [C.POINTER(i)] * 5,
+        "ouranos_rt_debug_nominal_form": [vp, i],
         "ouranos_rt_set_wait_limit": [vp, d],
         "ouranos_rt_debug_wait_bias": [vp, i],
         "ouranos_solve": [vp, i, i, i, d, vp, vp, vp, C.POINTER(SolveInfo)],

@@ -426,7 +426,7 @@ int ouranos_batch_create(const ouranos_problem_desc* descs, int count, int devic
       return OURANOS_ERR_UNSUPPORTED;
     }
     r->in_batch = true;
-    BR(member(b, p, ouranos_rt_set_tiling(r, 0, 0, 0)));  // the default form of a batch's member
+    BR(member(b, p, rt_set_tiling(r, 0, 0, 0)));  // the default form of a batch's member
   }
   b->device = b->rt[0]->device;
   for (ouranos_rt* r : b->rt)
@@ -575,6 +575,8 @@ int ouranos_batch_autotune(ouranos_batch* b, int precision, int reps, int* tilin
       auto it = g_tune_cache.find(key);
       if (it != g_tune_cache.end()) best = it->second;
     }
+    // (orders whose lanes share their cells whatever the tiling: nothing to time)
+    if (!per_lane_kernel(r->dim, r->p1)) best = {0, 0, 0};
     if (best.empty()) {
       std::vector<std::vector<int>> cand;
       if (r->dim == 2) cand = {{32, 1, 1}, {16, 1, 2}, {8, 1, 4}, {4, 1, 8}};
@@ -590,7 +592,7 @@ int ouranos_batch_autotune(ouranos_batch* b, int precision, int reps, int* tilin
       BC(cudaMemsetAsync(tx.p, 0, sizeof(double) * len, b->stream), "autotune");
       double best_ms = 1e30;
       for (const auto& c : cand) {
-        BR(member(b, (int)p, ouranos_rt_set_tiling(r, c[0], c[1], c[2])));
+        BR(member(b, (int)p, rt_set_tiling(r, c[0], c[1], c[2])));
         r->precision = precision;
         double t = 1e30;
         for (int k = 0; k <= reps; ++k) {  // first run warms up
@@ -608,7 +610,7 @@ int ouranos_batch_autotune(ouranos_batch* b, int precision, int reps, int* tilin
     }
     // rebuilding the schedule also clears the edge buffers of the single-
     // problem sweeps timed above
-    BR(member(b, (int)p, ouranos_rt_set_tiling(r, best[0], best[1], best[2])));
+    BR(member(b, (int)p, rt_set_tiling(r, best[0], best[1], best[2])));
     if (tiling_out)
       BR(member(b, (int)p, ouranos_rt_get_tiling(r, tiling_out + 3 * p, tiling_out + 3 * p + 1, tiling_out + 3 * p + 2)));
   }

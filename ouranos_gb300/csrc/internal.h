@@ -402,6 +402,7 @@ int rt_apply_device(ouranos_rt* rt, const double* x, double* y);
 // which must be current; once per device, called by ouranos_rt_create
 int noalloc_setup(int device);
 void nominal_tiling(const ouranos_rt* rt, int& wx, int& wy, int& lpc);
+int rt_set_tiling(ouranos_rt* rt, int cells_x, int cells_y, int dirs);
 // whether the default form may take warp tiles of wx x wy cells for values of
 // real_bytes: its scratch then holds the problem if the nominal tiling's did
 bool noalloc_fits(const ouranos_rt* rt, int wx, int wy, size_t real_bytes);
@@ -467,6 +468,7 @@ struct ouranos_rt {
   int wx = 0, wy = 1, kd = 0;          // 0 = not chosen yet
   int tiling[3] = {0, 0, 1};           // the tiling set by the caller (0: the default)
   int lpc = 1;                         // lanes per cell
+  bool nominal_form = false;           // test hook: the default is the nominal tiling's kernel
   bool in_batch = false;               // a member of a batch (default_tiling)
   bool grouped = false;                // the default form (sweep_group.cuh); wx, wy, lpc are its own
   int tiles_x = 0, tiles_y = 0, n_groups_dir = 0, n_tasks = 0;

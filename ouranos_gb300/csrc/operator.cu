@@ -302,6 +302,8 @@ size_t edge_bytes(const ouranos_rt* rt, int wx, int wy) {
 bool fp64_cell_solves(const ouranos_rt* rt) {
   return rt->fp64_contract == OURANOS_FP64_NATIVE || rt->fp64_contract == OURANOS_FP64_DF64;
 }
+int build_schedule(ouranos_rt* rt);
+int setup_group(ouranos_rt* rt);
 int default_tiling(ouranos_rt* rt) {
   rt->kd = 1;
   int wx0 = 0, wy0 = 0, lpc0 = 0;
@@ -324,6 +326,7 @@ int default_tiling(ouranos_rt* rt) {
     }
   }
   if (rt->n_mom == 2 && rt->n * 3 <= 32) lanes.clear();  // two fused moments: the per-lane form
+  if (rt->nominal_form && (per_lane_kernel(rt->dim, rt->p1) || lpc0 == 32)) lanes.clear();
   // FP64 cell solves: bound by the FP64 pipe, which wants few idle lanes and tiles
   // spread evenly (sweep kernel, ms, nominal / default form above: 2-D Q2 256^2 LS S16
   // 2.52 / 3.44, 3-D Q1 48^3 LS S8 2.74 / 2.87, 3-D Q3 12^3 LS S4 0.80 / 0.91; but 2-D Q2
@@ -361,6 +364,21 @@ int default_tiling(ouranos_rt* rt) {
   rt->wy = wy0;
   rt->lpc = lpc0;
   rt->grouped = false;
+  return OURANOS_OK;
+}
+
+// What the default depends on has changed: choose again, unless the caller set a tiling
+int choose_default_again(ouranos_rt* rt) {
+  if (rt->tiling[0]) return OURANOS_OK;
+  cudaSetDevice(rt->device);
+  const int wx = rt->wx, wy = rt->wy, lpc = rt->lpc;
+  const bool grouped = rt->grouped;
+  OK_OR_RETURN(default_tiling(rt));
+  if (wx == rt->wx && wy == rt->wy && lpc == rt->lpc && grouped == rt->grouped) return OURANOS_OK;
+  CU(cudaStreamSynchronize(rt->stream), "tiling");
+  OK_OR_RETURN(build_schedule(rt));
+  OK_OR_RETURN(setup_group(rt));
+  CU(cudaStreamSynchronize(rt->stream), "tiling");
   return OURANOS_OK;
 }
 
@@ -1145,6 +1163,45 @@ int rt_stage_out(ouranos_rt* rt, const double* dv, double* user) { return stage_
 int rt_result_target(ouranos_rt* rt, const double* in, double* user, bool in_place, DevBuf& buf, double** out) {
   return result_target(rt, in, user, in_place, buf, out);
 }
+// ouranos_rt_set_tiling, the nominal tiling being one like any other
+int rt_set_tiling(ouranos_rt* rt, int cells_x, int cells_y, int dirs) {
+  cudaSetDevice(rt->device);
+  // the layout of the inverse tables: the grouped forms' by their lanes, the
+  // transposed one of one warp per cell, or rows
+  auto layout = [&] { return rt->grouped ? 100 + rt->lpc : (rt->lpc == 32 ? 32 : 0); };
+  const int before = layout();
+  if (cells_x == 0 && cells_y == 0 && dirs == 0) {
+    OK_OR_RETURN(default_tiling(rt));
+    rt->tiling[0] = 0;
+  } else {
+    if (rt->dim == 2) cells_y = 1;
+    const int lanes = cells_x * cells_y * dirs;
+    const bool wide = lanes == 1;            // one warp per cell
+    const bool two = lanes == 16 && rt->n >= 9;  // two lanes per cell
+    if (cells_x < 1 || cells_y < 1 || dirs < 1 || (lanes != 32 && !two && !wide) || (dirs & (dirs - 1)))
+      return bad(rt, "tiling must satisfy cells_x*cells_y*dirs == 32 (or 16, two lanes per cell, for cells "
+                     "of 9 or more dofs; or 1 x 1 x 1, one warp per cell) with dirs a power of two");
+    if (!wide && !per_lane_order(rt->dim, rt->p1))
+      return bad(rt, "this DG order runs one warp per cell only (tiling 1 x 1 x 1): the per-lane sweep "
+                     "covers 2-D Q1..Q4 and 3-D Q1..Q2");
+    if (!wide && !per_lane_kernel(rt->dim, rt->p1)) {
+      OK_OR_RETURN(default_tiling(rt));  // these orders' lanes share their cells whatever the tiling
+    } else {
+      rt->wx = cells_x;
+      rt->wy = cells_y;
+      rt->kd = dirs;
+      rt->lpc = wide ? 32 : (two ? 2 : 1);
+      rt->grouped = false;
+    }
+    rt->tiling[0] = cells_x;
+    rt->tiling[1] = cells_y;
+    rt->tiling[2] = dirs;
+  }
+  OK_OR_RETURN(build_schedule(rt));
+  if (layout() != before) OK_OR_RETURN(setup_group(rt));  // the tables change layout
+  CU(cudaStreamSynchronize(rt->stream), "tiling");
+  return OURANOS_OK;
+}
 }  // namespace ouranos
 
 // ===================================================================== C-ABI
@@ -1390,18 +1447,7 @@ int ouranos_rt_set_fp64_contractions(ouranos_rt* rt, int mode) {
   const bool before = fp64_cell_solves(rt);
   rt->fp64_contract = mode;
   // the default form may be another one for FP64 cell solves
-  if (fp64_cell_solves(rt) != before && rt->tiling[0] == 0 && !rt->in_batch) {
-    cudaSetDevice(rt->device);
-    const int wx = rt->wx, wy = rt->wy, lpc = rt->lpc;
-    const bool grouped = rt->grouped;
-    OK_OR_RETURN(default_tiling(rt));
-    if (wx != rt->wx || wy != rt->wy || lpc != rt->lpc || grouped != rt->grouped) {
-      CU(cudaStreamSynchronize(rt->stream), "tiling");
-      OK_OR_RETURN(build_schedule(rt));
-      OK_OR_RETURN(setup_group(rt));
-      CU(cudaStreamSynchronize(rt->stream), "tiling");
-    }
-  }
+  if (fp64_cell_solves(rt) != before && !rt->in_batch) OK_OR_RETURN(choose_default_again(rt));
   return OURANOS_OK;
 }
 
@@ -1648,42 +1694,12 @@ int ouranos_rt_last_sweep_ms(const ouranos_rt* rt, double* ms, int* kernels) {
 
 int ouranos_rt_set_tiling(ouranos_rt* rt, int cells_x, int cells_y, int dirs) {
   if (!rt) return OURANOS_ERR_BAD_INPUT;
-  cudaSetDevice(rt->device);
-  // the layout of the inverse tables: the grouped forms' by their lanes, the
-  // transposed one of one warp per cell, or rows
-  auto layout = [&] { return rt->grouped ? 100 + rt->lpc : (rt->lpc == 32 ? 32 : 0); };
-  const int before = layout();
-  if (cells_x == 0 && cells_y == 0 && dirs == 0) {
-    OK_OR_RETURN(default_tiling(rt));
-    rt->tiling[0] = 0;
-  } else {
-    if (rt->dim == 2) cells_y = 1;
-    const int lanes = cells_x * cells_y * dirs;
-    const bool wide = lanes == 1;            // one warp per cell
-    const bool two = lanes == 16 && rt->n >= 9;  // two lanes per cell
-    if (cells_x < 1 || cells_y < 1 || dirs < 1 || (lanes != 32 && !two && !wide) || (dirs & (dirs - 1)))
-      return bad(rt, "tiling must satisfy cells_x*cells_y*dirs == 32 (or 16, two lanes per cell, for cells "
-                     "of 9 or more dofs; or 1 x 1 x 1, one warp per cell) with dirs a power of two");
-    if (!wide && !per_lane_order(rt->dim, rt->p1))
-      return bad(rt, "this DG order runs one warp per cell only (tiling 1 x 1 x 1): the per-lane sweep "
-                     "covers 2-D Q1..Q4 and 3-D Q1..Q2");
-    if (!wide && !per_lane_kernel(rt->dim, rt->p1)) {
-      OK_OR_RETURN(default_tiling(rt));  // these orders' lanes share their cells whatever the tiling
-    } else {
-      rt->wx = cells_x;
-      rt->wy = cells_y;
-      rt->kd = dirs;
-      rt->lpc = wide ? 32 : (two ? 2 : 1);
-      rt->grouped = false;
-    }
-    rt->tiling[0] = cells_x;
-    rt->tiling[1] = cells_y;
-    rt->tiling[2] = dirs;
-  }
-  OK_OR_RETURN(build_schedule(rt));
-  if (layout() != before) OK_OR_RETURN(setup_group(rt));  // the tables change layout
-  CU(cudaStreamSynchronize(rt->stream), "tiling");
-  return OURANOS_OK;
+  // the nominal tiling, which get_tiling reports of a default handle, is the default: a
+  // tiling that was read and set again keeps the form
+  int wx = 0, wy = 0, lpc = 0;
+  nominal_tiling(rt, wx, wy, lpc);
+  if (cells_x == wx && (rt->dim == 2 || cells_y == wy) && dirs == 1) cells_x = cells_y = dirs = 0;
+  return rt_set_tiling(rt, cells_x, cells_y, dirs);
 }
 
 int ouranos_rt_get_tiling(const ouranos_rt* rt, int* cx, int* cy, int* dirs) {
@@ -1694,6 +1710,22 @@ int ouranos_rt_get_tiling(const ouranos_rt* rt, int* cx, int* cy, int* dirs) {
   if (cy) *cy = wy;
   if (dirs) *dirs = rt->tiling[0] ? rt->tiling[2] : 1;
   return OURANOS_OK;
+}
+
+int ouranos_rt_get_form(const ouranos_rt* rt, int* cx, int* cy, int* dirs, int* lanes, int* default_form) {
+  if (!rt) return OURANOS_ERR_BAD_INPUT;
+  if (cx) *cx = rt->wx;
+  if (cy) *cy = rt->wy;
+  if (dirs) *dirs = rt->kd;
+  if (lanes) *lanes = rt->lpc;
+  if (default_form) *default_form = rt->grouped;
+  return OURANOS_OK;
+}
+
+int ouranos_rt_debug_nominal_form(ouranos_rt* rt, int on) {
+  if (!rt) return OURANOS_ERR_BAD_INPUT;
+  rt->nominal_form = on != 0;
+  return choose_default_again(rt);
 }
 
 int ouranos_rt_set_wait_limit(ouranos_rt* rt, double ns) {

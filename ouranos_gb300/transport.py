@@ -169,6 +169,16 @@ class RadiativeTransfer:
         self._check(_capi.lib().ouranos_rt_get_tiling(self._h, C.byref(a), C.byref(b), C.byref(c)))
         return a.value, b.value, c.value
 
+    def form(self):
+        """What the sweeps run: (cells_x, cells_y, dirs) of a warp's tile, the lanes
+        that share a cell, and whether it is one of the default forms."""
+        v = [C.c_int() for _ in range(5)]
+        self._check(_capi.lib().ouranos_rt_get_form(self._h, *map(C.byref, v)))
+        return tuple(k.value for k in v[:4]) + (bool(v[4].value),)
+
+    def debug_nominal_form(self, on):
+        self._check(_capi.lib().ouranos_rt_debug_nominal_form(self._h, int(on)))
+
     def set_stream(self, stream):
         """Run on a caller's cudaStream_t (an int handle, e.g. torch's
         ``torch.cuda.current_stream().cuda_stream``); None = own stream."""
