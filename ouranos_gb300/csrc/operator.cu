@@ -10,6 +10,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "form_rule.h"
 #include "internal.h"
 
 using namespace ouranos;
@@ -348,8 +349,8 @@ int default_tiling(ouranos_rt* rt) {
     // smaller tiles hand over more edges: not where these crowd out the angular
     // flux and the expanded source, nor where the allocation-free Apply would no
     // longer hold a problem it holds with the nominal tiling
-    if (H != 2 && edge_bytes(rt, wx, wy) > edge_bytes(rt, wx0, wy0) &&
-        edge_bytes(rt, wx, wy) + 16 * (size_t)rt->n_dir * rt->n_dofs > free_b / 2)
+    if (H != 2 && edges_crowd(edge_bytes(rt, wx, wy), edge_bytes(rt, wx0, wy0), 16 * (size_t)rt->n_dir * rt->n_dofs,
+                              free_b, rt->d_psi.bytes + rt->d_q.bytes + rt->d_edge_x.bytes + rt->d_edge_y.bytes))
       continue;
     bool fits = true;
     for (size_t rb : {4, 8}) fits = fits && noalloc_fits(rt, wx, wy, rb);
