@@ -293,10 +293,11 @@ extern "C" int ouranos_rt_apply_noalloc(ouranos_rt* rt, const double* x, double*
   // double, and the double-float pairs, take 8 bytes a value
   const size_t rb = rt->precision == OURANOS_FP64 ? 8 : 4;
   const Layout L = layout_for(rt, rt->wx, rt->wy, rb, 2 * rb, expand_source);
-  // what it takes is counted with the nominal tiling; the default form is only
-  // chosen where it needs no more room than there is (noalloc_fits)
-  const size_t nominal = nominal_bytes(rt, rb);
-  const size_t need = rt->grouped ? std::max(nominal, L.total) : L.total;
+  // what it takes is counted with two tagged words to an edge value in either
+  // precision, for a default form with the nominal tiling, which is only left where
+  // the smaller tiles need no more room than there is (noalloc_fits)
+  const size_t need = rt->grouped ? std::max(nominal_bytes(rt, rb), L.total)
+                                  : layout_for(rt, rt->wx, rt->wy, rb, 16, expand_source).total;
   if (need > kNoAllocScratchBytes) {
     char buf[256];
     std::snprintf(buf, sizeof buf,
