@@ -409,7 +409,7 @@ int ouranos_batch_create(const ouranos_problem_desc* descs, int count, int devic
   *out = b;  // kept on failure so the caller can read the message; it must destroy it
   for (int p = 0; p < count; ++p) {
     ouranos_rt* r = nullptr;
-    const int rc = ouranos_rt_create(&descs[p], device, &r);
+    const int rc = rt_create(&descs[p], device, true, &r);
     if (rc != OURANOS_OK) {
       char buf[512];
       std::snprintf(buf, sizeof buf, "problem %d: %s", p, r ? r->err.c_str() : "creation failed");
@@ -425,8 +425,6 @@ int ouranos_batch_create(const ouranos_problem_desc* descs, int count, int devic
       b->err = buf;
       return OURANOS_ERR_UNSUPPORTED;
     }
-    r->in_batch = true;
-    BR(member(b, p, rt_set_tiling(r, 0, 0, 0)));  // the default form of a batch's member
   }
   b->device = b->rt[0]->device;
   for (ouranos_rt* r : b->rt)

@@ -313,6 +313,9 @@ cudaError_t launch_axpby(double a, const double* x, double b, double* y, long le
 cudaError_t launch_multi_axpy(const double* const* V, int k, const double* coef, double scale,
                               double* w, long len, cudaStream_t s);
 cudaError_t launch_bump_epoch(unsigned* epoch, cudaStream_t s);
+// the columns' classes (each below 256), four planes to a word, for both sweep
+// directions: out[dir][plane / 4][column] of cls[plane][column]
+cudaError_t launch_pack_classes(const int* cls, unsigned* out, int planes, long columns, cudaStream_t s);
 cudaError_t launch_to_f32(const double* in, float* out, long n, cudaStream_t s);
 cudaError_t launch_to_f32_pairs(const df64* in, float* out, long n, cudaStream_t s);
 // q[d][c n + i] += inv_vdt sum_j M_ij psi[d][c n + j]  (implicit Euler's psi^n term)
@@ -403,6 +406,7 @@ int rt_apply_device(ouranos_rt* rt, const double* x, double* y);
 int noalloc_setup(int device);
 void nominal_tiling(const ouranos_rt* rt, int& wx, int& wy, int& lpc);
 int rt_set_tiling(ouranos_rt* rt, int cells_x, int cells_y, int dirs);
+int rt_create(const ouranos_problem_desc* D, int device, bool in_batch, ouranos_rt** out);
 // whether the default form may take warp tiles of wx x wy cells for values of
 // real_bytes: its scratch then holds the problem if the nominal tiling's did
 bool noalloc_fits(const ouranos_rt* rt, int wx, int wy, size_t real_bytes);
@@ -479,7 +483,7 @@ struct ouranos_rt {
   std::vector<double> class_abs_omega;  // [n_dir_class][3]
   int n_dir_class = 0;
   std::vector<double> sigma_class_value; // per sigma_t class
-  std::vector<int> cell_class_h;
+  std::vector<int> mat_class_h;         // sigma_t class of each material, as in d_cell_class
   long long wait_limit_ns = 2000000000LL;
   int wait_bias = 0;
   unsigned epoch = 0;                  // sweep counter, tags edge-buffer words

@@ -207,6 +207,9 @@ bool tables_spill(const ouranos_rt* rt, size_t real_bytes) {
   return rt->n_queues > 1 && table * rt->n_dir_class > (64u << 10);
 }
 
+template <typename real>
+std::vector<unsigned char> group_face_table(const FETables& fe, int H);
+
 int build_schedule(ouranos_rt* rt) {
   const int dim = rt->dim;
   const int NX = rt->nx[0], NY = dim == 3 ? rt->nx[1] : 1, NS = rt->nx[dim - 1];
@@ -253,6 +256,11 @@ int build_schedule(ouranos_rt* rt) {
     }
     OK_OR_RETURN(upload(rt, rt->d_queue_tasks, by_class, "tasks"));
     OK_OR_RETURN(upload(rt, rt->d_queue_first, first, "tasks"));
+  }
+  if (rt->grouped && rt->lpc > 1) {
+    OK_OR_RETURN(upload(rt, rt->d_fgroup64, group_face_table<double>(rt->fe, rt->lpc), "face tables"));
+    OK_OR_RETURN(upload(rt, rt->d_fgroupdf, group_face_table<df64>(rt->fe, rt->lpc), "face tables"));
+    OK_OR_RETURN(upload(rt, rt->d_fgroup32, group_face_table<float>(rt->fe, rt->lpc), "face tables"));
   }
   OK_OR_RETURN(upload(rt, rt->d_group_dirs, gdirs, "group dirs"));
   OK_OR_RETURN(upload(rt, rt->d_group_flip, gflip, "group flips"));
@@ -389,33 +397,43 @@ int choose_default_again(ouranos_rt* rt) {
 // lone rows, [16-byte piece of columns][lane]; the rest is zero
 template <typename real>
 std::vector<unsigned char> group_tables(const std::vector<double>& ainv, size_t mats, int dim, int p1, int H) {
+  constexpr bool df = std::is_same<real, df64>::value;
   const int n = dim == 2 ? p1 * p1 : p1 * p1 * p1, sz = (int)sizeof(real);
   const bool adj = p1 % 2 == 0 && (n / 2) % H == 0;
   const int R = (n + H - 1) / H, RP = R / 2;
   const int pj = 8 / sz, ncp = (n + pj - 1) / pj, pl = 16 / sz, ncl = R % 2 ? (n + pl - 1) / pl : 0;
   const size_t bytes = (size_t)16 * H * (RP * ncp + ncl);
+  // where entry (i, j) goes: its (high) part, and the low part of a double-float
+  // 8 bytes on in a pair, 4 in a lone row
+  std::vector<int> at((size_t)n * n);
+  std::vector<char> pair(n);
+  for (int h = 0; h < H; ++h)
+    for (int k = 0; k < R; ++k) {
+      const int i = adj ? 2 * (h + H * (k / 2)) + k % 2 : h + H * k;
+      if (i >= n) continue;
+      pair[i] = k / 2 < RP;
+      for (int j = 0; j < n; ++j)
+        at[(size_t)i * n + j] = pair[i] ? (((k / 2) * ncp + j / pj) * H + h) * 16 + (j % pj) * 2 * sz + (df ? 4 : sz) * (k % 2)
+                                        : (RP * ncp * H + (j / pl) * H + h) * 16 + (j % pl) * sz;
+    }
   std::vector<unsigned char> out(mats * bytes, 0);
-  for (size_t m = 0; m < mats; ++m)
-    for (int h = 0; h < H; ++h)
-      for (int k = 0; k < R; ++k) {
-        const int i = adj ? 2 * (h + H * (k / 2)) + k % 2 : h + H * k;
-        if (i >= n) continue;
-        for (int j = 0; j < n; ++j) {
-          const double v = ainv[(m * n + i) * n + j];
-          unsigned char* at = out.data() + m * bytes;
-          const bool pair = k / 2 < RP;
-          if (pair) at += ((size_t)((k / 2) * ncp + j / pj) * H + h) * 16 + (j % pj) * 2 * sz;
-          else at += ((size_t)RP * ncp * H + (size_t)(j / pl) * H + h) * 16 + (j % pl) * sz;
-          if constexpr (std::is_same<real, df64>::value) {
-            const df64 w = df64_split(v);
-            std::memcpy(at + (pair ? 4 * (k % 2) : 0), &w.hi, 4);
-            std::memcpy(at + (pair ? 8 + 4 * (k % 2) : 4), &w.lo, 4);
-          } else {
-            const real w = (real)v;
-            std::memcpy(at + (pair ? sz * (k % 2) : 0), &w, sz);
-          }
+  for (size_t m = 0; m < mats; ++m) {
+    const double* from = &ainv[m * n * n];
+    unsigned char* to = out.data() + m * bytes;
+    for (int i = 0; i < n; ++i)
+      for (int j = 0; j < n; ++j) {
+        unsigned char* p = to + at[(size_t)i * n + j];
+        const double v = from[(size_t)i * n + j];
+        if constexpr (df) {
+          const df64 w = df64_split(v);
+          std::memcpy(p, &w.hi, 4);
+          std::memcpy(p + (pair[i] ? 8 : 4), &w.lo, 4);
+        } else {
+          const real w = (real)v;
+          std::memcpy(p, &w, sz);
         }
       }
+  }
   return out;
 }
 
@@ -475,22 +493,25 @@ int setup_group(ouranos_rt* rt) {
     }
   }
   rt->sigma_class_value = cls_val;
-  std::vector<int> ccls(rt->n_cells);
-  for (long c = 0; c < rt->n_cells; ++c) ccls[c] = mat_cls[rt->material_id[c]];
-  OK_OR_RETURN(upload(rt, rt->d_cell_class, ccls, "cell classes"));
+  // (the cells' classes stay where the materials map to the same ones)
+  const bool same_map = mat_cls == rt->mat_class_h;
+  std::vector<int> ccls;
+  if (!same_map) {
+    ccls.resize(rt->n_cells);
+    for (long c = 0; c < rt->n_cells; ++c) ccls[c] = mat_cls[rt->material_id[c]];
+    rt->mat_class_h.clear();
+    rt->cls4_ok = false;
+    OK_OR_RETURN(upload(rt, rt->d_cell_class, ccls, "cell classes"));
+    rt->mat_class_h = mat_cls;
+  }
   // the columns' classes, four planes to a word, for either sweep direction
+  const bool had_cls4 = rt->cls4_ok;
   rt->cls4_ok = rt->grouped && rt->lpc == 1 && cls_val.size() <= 256;
-  if (rt->cls4_ok) {
-    const long NS = rt->nx[rt->dim - 1], ncol = rt->n_cells / NS, words = (NS + 3) / 4;
-    std::vector<unsigned> packed((size_t)2 * words * ncol, 0u);
-    for (int dir = 0; dir < 2; ++dir)
-      for (long k = 0; k < NS; ++k) {
-        unsigned* to = &packed[((size_t)dir * words + k / 4) * ncol];
-        const int* from = &ccls[ncol * (dir ? NS - 1 - k : k)];
-        const int shift = 8 * (int)(k % 4);
-        for (long c = 0; c < ncol; ++c) to[c] |= (unsigned)from[c] << shift;
-      }
-    OK_OR_RETURN(upload(rt, rt->d_cls4, packed, "cell classes"));
+  if (rt->cls4_ok && !had_cls4) {
+    const int NS = rt->nx[rt->dim - 1];
+    const long ncol = rt->n_cells / NS;
+    CU(rt->d_cls4.alloc(sizeof(unsigned) * 2 * ((NS + 3) / 4) * ncol), "cell classes");
+    CU(launch_pack_classes(rt->d_cell_class.as<int>(), rt->d_cls4.as<unsigned>(), NS, ncol, rt->stream), "cell classes");
   }
   // A'^-1 per (sigma class, |Omega| class)
   const size_t nn = (size_t)n * n;
@@ -505,11 +526,6 @@ int setup_group(ouranos_rt* rt) {
   std::vector<double> ainv_p;
   if (rt->grouped) {
     const size_t mats = cls_val.size() * rt->n_dir_class;
-    if (rt->lpc > 1) {
-      OK_OR_RETURN(upload(rt, rt->d_fgroup64, group_face_table<double>(rt->fe, rt->lpc), "face tables"));
-      OK_OR_RETURN(upload(rt, rt->d_fgroupdf, group_face_table<df64>(rt->fe, rt->lpc), "face tables"));
-      OK_OR_RETURN(upload(rt, rt->d_fgroup32, group_face_table<float>(rt->fe, rt->lpc), "face tables"));
-    }
     OK_OR_RETURN(upload(rt, rt->d_ainv64, group_tables<double>(ainv, mats, rt->dim, rt->p1, rt->lpc), "inverse tables"));
     OK_OR_RETURN(upload(rt, rt->d_ainvdf, group_tables<df64>(ainv, mats, rt->dim, rt->p1, rt->lpc), "inverse tables"));
     OK_OR_RETURN(upload(rt, rt->d_ainv32, group_tables<float>(ainv, mats, rt->dim, rt->p1, rt->lpc), "inverse tables"));
@@ -1203,12 +1219,8 @@ int rt_set_tiling(ouranos_rt* rt, int cells_x, int cells_y, int dirs) {
   CU(cudaStreamSynchronize(rt->stream), "tiling");
   return OURANOS_OK;
 }
-}  // namespace ouranos
-
-// ===================================================================== C-ABI
-extern "C" {
-
-int ouranos_rt_create(const ouranos_problem_desc* D, int device, ouranos_rt** out) {
+// ouranos_rt_create; in_batch: for a member of a batch (default_tiling)
+int rt_create(const ouranos_problem_desc* D, int device, bool in_batch, ouranos_rt** out) {
   if (!out) return OURANOS_ERR_BAD_INPUT;
   *out = nullptr;
   if (!D) return OURANOS_ERR_BAD_INPUT;
@@ -1237,6 +1249,7 @@ int ouranos_rt_create(const ouranos_problem_desc* D, int device, ouranos_rt** ou
   if (device < 0) cudaGetDevice(&device);
   rt->device = device;
   if (cudaSetDevice(device) != cudaSuccess) return fail(cuda_fail(rt, cudaGetLastError(), "set device"));
+  rt->in_batch = in_batch;
   rt->dim = D->dim;
   rt->p = D->fe_order;
   rt->p1 = rt->p + 1;
@@ -1397,6 +1410,14 @@ int ouranos_rt_create(const ouranos_problem_desc* D, int device, ouranos_rt** ou
     return fail(cuda_fail(rt, cudaGetLastError(), "setup"));
   *out = rt;
   return OURANOS_OK;
+}
+}  // namespace ouranos
+
+// ===================================================================== C-ABI
+extern "C" {
+
+int ouranos_rt_create(const ouranos_problem_desc* D, int device, ouranos_rt** out) {
+  return rt_create(D, device, false, out);
 }
 
 int ouranos_rt_destroy(ouranos_rt* rt) {
