@@ -624,8 +624,25 @@ __device__ __forceinline__ void sweep_group_task(const SweepArgs<real>& a, const
   }
 }
 
+// Resident blocks per SM the registers are cut for (0: the compiler's choice).  Left to
+// itself the compiler settled on anything between 64 and 168 registers, another number
+// after every change around the loops, and the loads of the tables run ahead as far as
+// there are registers: with three blocks they do.  Sweep kernel, double-float / FP32,
+// us, the compiler's choice -> 3 blocks (4 in FP32 up to 16 dofs):
+//   2-D Q3 135x93 LS S12  466 / 235 -> 446 / 223    2-D Q4 100^2 S8, 16 materials  954 / 346 -> 653 / 264
+//   2-D Q5 64^2 LS S8, 16 materials  731 / 252 -> 488 / 192
+//   3-D Q2 24^3 LS S6     636 / 243 -> 581 / 238    3-D Q3 16^3 S4, 16 materials   956 / 247 -> 556 / 169
+//   3-D Q4 10^3 LS S4     522 / 163 -> 491 / 110    3-D Q5 8^3 S4                  837 / 536 -> 735 / 227
+// (five blocks: 3-D Q5 2345 / 424; FP32 3-D Q2 48^3 S8 with 8 lanes is the one exception,
+// 2233 -> 2390).
+template <typename real, int DIM, int P1, int H>
+constexpr int group_blocks() {
+  constexpr int N = Cell<DIM, P1>::N;
+  if (sizeof(real) == 4 && N == 27 && H == 8) return 0;
+  return sizeof(real) == 4 && N <= 16 ? 4 : 3;
+}
 template <typename real, int DIM, int P1, int FM, int H>
-__global__ void __launch_bounds__(128) sweep_group_kernel(const __grid_constant__ SweepArgs<real> a) {
+__global__ void __launch_bounds__(128, (group_blocks<real, DIM, P1, H>())) sweep_group_kernel(const __grid_constant__ SweepArgs<real> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr unsigned FULL = 0xffffffffu;
   // With queues, an SM starts on one |Omega| class, whose tables its L1 then holds, and
@@ -678,7 +695,7 @@ struct BatchLaunch {
 
 // Many problems in one persistent launch (see sweep_batch_kernel)
 template <typename real, int DIM, int P1, int FM, int H>
-__global__ void __launch_bounds__(128) sweep_group_batch_kernel(const SweepArgs<real>* __restrict__ args,
+__global__ void __launch_bounds__(128, (group_blocks<real, DIM, P1, H>())) sweep_group_batch_kernel(const SweepArgs<real>* __restrict__ args,
                                                                 const int2* __restrict__ tmap, int n_total, int* ticket,
                                                                 const int* status, const unsigned* epoch) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -694,8 +711,7 @@ __global__ void __launch_bounds__(128) sweep_group_batch_kernel(const SweepArgs<
 // L1 kept beside the resident blocks, for the inverse tables of the running
 // directions: the sources stream past it (16-byte cp.async.cg), and 28, 64 and
 // 112 KB measured the same within the spread; more where an SM's warps share one
-// class's tables (3-D Q3 20x17x23, us, 64 / 100 / 132 / 164 KB: 1294 / 1193 / 1167 / 1170;
-// 3-D Q2 37x29x41: 2102 / 2095 / 2108 / 2400)
+// class's tables
 constexpr int kGroupKeepKb = 64, kQueueKeepKb = 132;
 
 template <typename real, int DIM, int P1, int FM, int H>
