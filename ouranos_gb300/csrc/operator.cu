@@ -198,10 +198,17 @@ int build_symmetry(ouranos_rt* rt) {
 constexpr int kQueueTickets = 2, kMaxQueues = 48;
 
 // Whether the inverse tables of all |Omega| classes are more than an SM's L1 keeps
-// beside the slots, so that its warps should work on one class at a time.  Apply, us,
-// one queue / a queue per class / with 132 KB of L1 kept for it (kGroupKeepKb):
-// 3-D Q3 20x17x23 LS S4, two materials (32 KB a table) 1342 / 1294 / 1167, the larger L1
-// alone 1396; 3-D Q2 37x29x41 LS S6 (6 KB a table) 2152 / 2102 / 2108.
+// beside the slots, so that its warps should work on one class at a time.  Sweep
+// kernel, double-float / FP32, us, one queue -> a queue per class (materials drawn
+// cell by cell):
+//   2-D Q3 135x93 LS S12   2 materials 458 / 225 -> 442 / 223   16  485 / 243 -> 452 / 223
+//   2-D Q3 300^2 LS S8     2          1343 / 592 -> 1343 / 592  16 1413 / 628 -> 1324 / 592
+//   2-D Q4 200^2 LS S12    2          2000 / 692 -> 1886 / 690  16 2179 / 1007 -> 2048 / 862
+//   2-D Q5 64^2 LS S16     2           751 / 270 -> 702 / 257   16  794 / 350 -> 769 / 319
+//   3-D Q2 48^3 LS S8      2          6251 / 2234 -> 5958 / 2233  16 6611 / 2833 -> 6403 / 2341
+//   3-D Q3 16^3 LS S4      2           556 / 137 -> 538 / 139   16  557 / 163 -> 550 / 169
+//   3-D Q3 20x17x23 LS S8  2          2087 / 600 -> 2091 / 542  16 2098 / 618 -> 2100 / 670
+//   3-D Q5 8^3 LS S4       1           825 / 218 -> 737 / 229    4  825 / 223 -> 741 / 225
 bool tables_spill(const ouranos_rt* rt, size_t real_bytes) {
   const size_t table = real_bytes * rt->n * rt->n * rt->sigma_class_value.size();
   return rt->n_queues > 1 && table * rt->n_dir_class > (64u << 10);

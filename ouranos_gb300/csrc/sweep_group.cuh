@@ -649,11 +649,11 @@ __global__ void __launch_bounds__(128, (group_blocks<real, DIM, P1, H>())) sweep
   // goes on to the next when that has no tasks left.  Every queue is in dependency
   // order and a class's tasks wait on none of another's, so any warp may take the
   // head of any queue.
-  int queue = 0, left = a.n_queues;
-  if (left > 1) {
+  int queue = 0;
+  if (a.n_queues > 1) {
     unsigned sm;
     asm("mov.u32 %0, %%smid;" : "=r"(sm));
-    queue = (int)(sm % (unsigned)left);
+    queue = (int)(sm % (unsigned)a.n_queues);
   }
   for (;;) {
     int task = 0, stop = 0;
@@ -671,8 +671,21 @@ __global__ void __launch_bounds__(128, (group_blocks<real, DIM, P1, H>())) sweep
       task += first;
     }
     if (task >= count) {
-      if (--left == 0) return;
-      queue = queue + 1 == a.n_queues ? 0 : queue + 1;
+      if (a.n_queues <= 1) return;
+      // the next queue with tasks left, from all counters at once (asking one after the
+      // other cost an atomic each, of every idle warp: 2-D Q3 64^2 LS S16 FP32, 36
+      // queues, 233 us where one queue takes 125)
+      const int lane = threadIdx.x & 31;
+      unsigned long long open = 0;
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+        const int k = 32 * part + lane;
+        const bool some = k < a.n_queues && *(volatile int*)(a.ticket + k) < a.queue_first[k + 1] - a.queue_first[k];
+        open |= (unsigned long long)__ballot_sync(FULL, some) << 32 * part;
+      }
+      if (!open) return;
+      const unsigned long long after = open >> queue >> 1 << 1 << queue;
+      queue = __ffsll((long long)(after ? after : open)) - 1;
       continue;
     }
     sweep_group_task<real, DIM, P1, FM, H>(a, task, smem_raw);

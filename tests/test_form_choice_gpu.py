@@ -99,3 +99,32 @@ def test_autotuned_tilings_of_orders_that_choose_their_lanes():
     probs = [_problem(og, 2, 3, (9, 5)), _problem(og, 2, 4, (5, 4)), _problem(og, 3, 2, (5, 3, 4))]
     with og.Batch(probs) as b:
         assert b.autotune(reps=1).tolist() == [[16, 1, 1], [16, 1, 1], [4, 4, 1]]
+
+
+# (problem, directions' |Omega| classes): a task queue per class, below and above a warp's 32
+@pytest.mark.parametrize("dim,order,n,sn,mats", [(2, 3, (17, 5), 16, 64), (2, 4, (9, 4), 16, 16), (2, 5, (5, 4), 16, 8),
+                                                 (3, 2, (5, 4, 3), 8, 16), (3, 3, (3, 2, 2), 4, 4)])
+def test_task_queues_give_one_warp_per_cells_bits(dim, order, n, sn, mats):
+    import ouranos_gb300 as og
+    rng = np.random.default_rng(dim + order)
+    q = og.build_quadrature("LS", sn, 1, dim=dim)
+    nc = int(np.prod(n))
+    p = og.Problem(dim, order, n, (0.0,) * dim, (1.0,) * dim, q, rng.uniform(0.5, 5.0, (mats, 1)),
+                   rng.uniform(0.0, 0.2, (mats, 1, 1, 2)), rng.integers(0, mats, nc).astype(np.int32),
+                   np.zeros(nc, np.int32), np.ones((1, 1)), (1,) * (2 * dim), np.ones((2 * dim, 1)))
+    x = rng.standard_normal(p.vector_length)
+    with og.RadiativeTransfer(p) as rt:
+        for precision in ("fp64", "fp32"):
+            rt.set_precision(precision)
+            rt.set_tiling()
+            assert rt.form()[4] and rt.form()[3] > 1
+            y, b = [rt.apply(x) for _ in range(3)], rt.rhs()
+            if (dim, order) in ((2, 3), (2, 4), (3, 2)):
+                rt.set_tiling(1, 1, 1)
+            else:
+                rt.debug_nominal_form(1)
+            assert rt.form()[3:] == (32, False)
+            ref = rt.apply(x)
+            assert all(np.array_equal(v, ref) for v in y)
+            assert np.array_equal(b, rt.rhs())
+            rt.debug_nominal_form(0)
