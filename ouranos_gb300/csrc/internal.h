@@ -93,7 +93,7 @@ inline bool per_lane_kernel(int dim, int p1) { return dim == 2 ? p1 <= 3 : p1 ==
 constexpr size_t kSrcSlack = 32;
 // Arguments of one sweep launch (see sweep.cuh for the algorithm).
 template <typename real>
-struct SweepArgs {
+struct TaskArgs {
   int nx, ny, nz;              // cells per axis (physical)
   int n_sweep;                 // cells along the sweep axis (y in 2-D, z in 3-D)
   long n_dofs;                 // cells * n
@@ -129,6 +129,10 @@ struct SweepArgs {
   int lpc;                     // lanes per cell: 1, 2 (cells of 9 or more dofs), or 32 (one warp
                                // per cell, sweep_wide.cuh; tiling 1 x 1 x 1, expanded source)
   int grouped;                 // 1: the default form, lpc lanes per cell (sweep_group.cuh)
+};
+// the same with what only the default forms read
+template <typename real>
+struct SweepArgs : TaskArgs<real> {
   int n_queues;                // more than 1 (grouped, lpc > 1): tasks come in queues, queue k's entries
   const int* queue_first;      // [queue_first[k], queue_first[k + 1]), each with a counter of its own at ticket[k]
   float minus_zero;            // -0, an addend the compiler does not know (pack2.cuh)

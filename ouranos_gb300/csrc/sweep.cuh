@@ -432,7 +432,7 @@ __device__ __forceinline__ real cell_row(const real (&xr)[NR], int r, int half) 
 // then covers 32 / H cells, so twice as many warps share the wavefront and
 // each does half the cell-solve arithmetic per step.
 template <typename real, int DIM, int P1, int FM, int H>
-__device__ __forceinline__ void sweep_task(const SweepArgs<real> a, const int task,
+__device__ __forceinline__ void sweep_task(const TaskArgs<real> a, const int task,
                                            unsigned char* smem_raw) {
   using C = Cell<DIM, P1>;
   constexpr int N = C::N;
@@ -865,7 +865,7 @@ __device__ __forceinline__ void sweep_task(const SweepArgs<real> a, const int ta
 // task a warp waits on was taken earlier by a running warp -- any grid is
 // deadlock-free.
 template <typename real, int DIM, int P1, int FM, int H>
-__global__ void __launch_bounds__(128) sweep_kernel(const SweepArgs<real> a) {
+__global__ void __launch_bounds__(128) sweep_kernel(const TaskArgs<real> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr unsigned FULL = 0xffffffffu;
   for (;;) {

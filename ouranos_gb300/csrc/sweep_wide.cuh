@@ -46,7 +46,7 @@ __device__ __forceinline__ real face_dot(const real* row, const real* up) {
 }
 
 template <typename real, int DIM, int P1>
-__device__ __forceinline__ void sweep_wide_task(const SweepArgs<real>& a, const int task,
+__device__ __forceinline__ void sweep_wide_task(const TaskArgs<real>& a, const int task,
                                                 unsigned char* smem_raw) {
   using C = Cell<DIM, P1>;
   using A = Arith<real>;
@@ -215,7 +215,7 @@ __device__ __forceinline__ void sweep_wide_task(const SweepArgs<real>& a, const 
 }
 
 template <typename real, int DIM, int P1>
-__global__ void __launch_bounds__(128) sweep_wide_kernel(const SweepArgs<real> a) {
+__global__ void __launch_bounds__(128) sweep_wide_kernel(const TaskArgs<real> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr unsigned FULL = 0xffffffffu;
   for (;;) {
