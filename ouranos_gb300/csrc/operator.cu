@@ -779,7 +779,14 @@ int sweep_launch(ouranos_rt* rt, SweepArgs<real>& a, int fm) {
   const int block = 128;
   // tasks are handed out by ticket, so any grid is deadlock-free; 8 blocks of
   // 4 warps per SM covers every instantiation's register budget
-  const int grid = std::min((rt->n_tasks + 3) / 4, std::max(1, sms * 8));
+  int grid = std::min((rt->n_tasks + 3) / 4, std::max(1, sms * 8));
+  // FP64 cell solves with one lane to a cell (2-D Q1): two blocks saturate an SM's FP64
+  // pipe, and a block more on some SMs only makes these the slowest.  Native FP64 sweep,
+  // us, all blocks / at most two an SM, nominal tiling's kernel: 256^2 LS S16 1140 / 1140,
+  // 1065; 300^2 S16 1902 / 1466, 1650; 400^2 S16 3036 / 2110, 2540; 600^2 S8 2620 / 2100,
+  // 2500; 700^2 S16 6136 / 5101, 6300.
+  if (std::is_same<real, double>::value && rt->grouped && rt->lpc == 1 && grid > sms)
+    grid = grid >= 2 * sms ? 2 * sms : (grid - sms < sms / 2 ? sms : grid);
   CU(cudaEventRecord(rt->ev0, rt->stream), "event");
   CU(launch_sweep<real>(rt->dim, rt->p1, fm, a, grid, block, rt->stream), "sweep launch");
   CU(cudaEventRecord(rt->ev1, rt->stream), "event");
