@@ -315,6 +315,28 @@ size_t edge_bytes(const ouranos_rt* rt, int wx, int wy) {
 // batch counts as a large problem: the batch's launch is full anyway, and fewer
 // forms are fewer launches.  Two lanes to a cell have the nominal tiling's tiles:
 // the last resort of the orders without a per-lane kernel.
+//
+// With one lane to a cell, a warp reads as many inverse tables at a time as its 32 cells
+// have materials, with four lanes an eighth of the cells.  Apply of 2-D Q2, P1, us,
+// double-float / FP32, 1 lane -> 4 lanes, by materials drawn cell by cell: 256^2 LS S16
+// 2: 1384 / 649 -> 1599 / 761, 4: 1447 / 777 -> 1649 / 782, 8: 1719 / 966 -> 1694 / 807,
+// 16: 1975 / 1137 -> 1766 / 841; 200^2 S8 2: 658 / 374 -> 710 / 417, 8: 698 / 415 ->
+// 739 / 436, 16: 773 / 447 -> 742 / 445; 500x400 S8 8: 2074 / 1138 -> 2032 / 1128.  With few
+// cells side by side the shorter step of four lanes counts more: 40^2 S16, 2 materials,
+// 201 / 132 -> 177 / 122, 64^2 S16 239 / 141 -> 269 / 166.
+double materials_per_row_tile(const ouranos_rt* rt) {
+  const long nx = rt->nx[0], rows = rt->n_cells / nx, tiles = (nx + 31) / 32;
+  std::vector<long> seen(rt->n_mat, -1);
+  long count = 0;
+  for (long r = 0; r < rows; ++r)
+    for (long t = 0; t < tiles; ++t)
+      for (long x = 32 * t; x < std::min(nx, 32 * t + 32); ++x) {
+        long& s = seen[rt->material_id[r * nx + x]];
+        count += s != r * tiles + t;
+        s = r * tiles + t;
+      }
+  return (double)count / (double)(rows * tiles);
+}
 bool fp64_cell_solves(const ouranos_rt* rt) {
   return rt->fp64_contract == OURANOS_FP64_NATIVE || rt->fp64_contract == OURANOS_FP64_DF64;
 }
@@ -329,7 +351,11 @@ int default_tiling(ouranos_rt* rt) {
   if (rt->dim == 2) {
     switch (rt->p1) {
       case 2: lanes = {1}; break;
-      case 3: lanes = rt->n_dir * tiles_x < 256 && !rt->in_batch ? std::vector<int>{4, 1} : std::vector<int>{1}; break;
+      case 3:
+        lanes = !rt->in_batch && (rt->n_dir * tiles_x < 256 || (long)rt->n_dir * rt->nx[0] < 200 * 32 ||
+                                  (!fp64_cell_solves(rt) && materials_per_row_tile(rt) > 6.0))
+                    ? std::vector<int>{4, 1} : std::vector<int>{1};
+        break;
       case 4: case 5: lanes = {8, 2}; break;
       default: lanes = {16}; break;
     }

@@ -28,7 +28,7 @@ def _set(rt, arith):
 
 
 # (problem, the default form's lanes per cell)
-FORMS = [((2, 1, (33, 9)), 1), ((2, 2, (9, 5)), 4), ((2, 2, (34, 6), 16), 1), ((2, 3, (9, 5)), 8), ((2, 4, (5, 4)), 8),
+FORMS = [((2, 1, (33, 9)), 1), ((2, 2, (9, 5)), 4), ((2, 2, (66, 6), 16), 1), ((2, 3, (9, 5)), 8), ((2, 4, (5, 4)), 8),
          ((2, 5, (4, 3)), 16), ((3, 1, (5, 9, 7)), 1), ((3, 2, (5, 3, 4)), 16), ((3, 3, (3, 2, 3)), 16),
          ((3, 4, (2, 2, 3)), 32), ((3, 5, (2, 1, 2), 2), 32)]
 
@@ -128,3 +128,24 @@ def test_task_queues_give_one_warp_per_cells_bits(dim, order, n, sn, mats):
             assert all(np.array_equal(v, ref) for v in y)
             assert np.array_equal(b, rt.rhs())
             rt.debug_nominal_form(0)
+
+
+def test_many_materials_side_by_side_share_cells():
+    """2-D Q2: four lanes to a cell where a row of 32 cells meets many materials, in any
+    order, one lane where they come in blocks; the same bits."""
+    import ouranos_gb300 as og
+    rng = np.random.default_rng(8)
+    q = og.build_quadrature("LS", 16, 1, dim=2)
+    n = (66, 5)
+    cells = np.arange(n[0] * n[1])
+    x = None
+    for mat, lanes in ((cells % 16, 4), (rng.integers(0, 16, cells.size), 4), (cells % 66 // 6, 1), (cells % 2, 1)):
+        p = og.Problem(2, 2, n, (0.0, 0.0), (1.0, 1.0), q, rng.uniform(0.5, 5.0, (16, 1)),
+                       rng.uniform(0.0, 0.2, (16, 1, 1, 2)), mat.astype(np.int32), np.zeros(cells.size, np.int32),
+                       np.ones((1, 1)), (1,) * 4, np.ones((4, 1)))
+        x = rng.standard_normal(p.vector_length)
+        with og.RadiativeTransfer(p) as rt:
+            assert rt.form()[3:] == (lanes, True)
+            y, b = rt.apply(x), rt.rhs()
+            rt.debug_nominal_form(1)
+            assert np.array_equal(rt.apply(x), y) and np.array_equal(rt.rhs(), b)
