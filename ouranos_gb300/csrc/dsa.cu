@@ -24,14 +24,17 @@
 // The diffusion system (one unknown per vertex, 27-point stencil in 3-D, its
 // coefficients assembled once per table rebuild) is solved approximately by
 // a fixed number of Jacobi-preconditioned conjugate-gradient steps, in FP32
-// with FP64 scalars, all in one cooperative launch (the vertex vectors of a
-// 64^3 mesh, 1.1 MB each, stay in L2) with two grid barriers per step:
+// with FP64 scalars (the threads' FP32 sums are added at FP64 accuracy), all in one
+// cooperative launch.  Where a thread holds few vertices the vectors and the stencil
+// rows stay on chip (dsa_cg_resident_kernel), else the vectors are in global memory
+// and L2.  The blocks meet once for the right-hand side's cell moments, once for
+// r.z, and twice per step:
 //   matvec : w = C z, p = z + beta p, q = w + beta q, pq = p.q, alpha = rz/pq
 //   update : x += alpha p, r -= alpha q, z = r / diag, rz' = r.z, beta = rz'/rz
 // (q = C p is carried by recurrence, so the matrix is applied once per step).
 // A caller may start the CG from a guess of f (the learned preconditioner's
 // prediction): it is first scaled to its energy-norm-optimal multiple, one
-// more grid barrier, so a poor guess can never start the CG farther from the
+// more meeting, so a poor guess can never start the CG farther from the
 // solution than zero does.
 // Every block sums the per-block partials of a dot product in block order, so
 // all blocks hold the same, deterministic scalars.
@@ -425,8 +428,8 @@ __device__ __forceinline__ void write_out(const DsaGeom& g, const double* v, dou
 // need no synchronisation; z of the neighbours and the partials cross
 // blocks, and the barrier's release/acquire fences order them (plain loads
 // after it see every write made before it).  Every block of the grid passes
-// the same 2 iters grid barriers.  Dot products: FP32 per thread, FP64 from
-// the block sums on; part_a/part_b hold the problem's nb partials.
+// the same 2 iters + 1 meetings (and one with a guess).  Dot products: FP32 per
+// thread, added at FP64 accuracy (meet); part_a/part_b hold the problem's nb partials.
 template <int DIM>
 __device__ __forceinline__ void cg_body(const DsaGeom& g, const float4* __restrict__ cell,
                                         const float* __restrict__ coef, const double* v, double* out, long len,

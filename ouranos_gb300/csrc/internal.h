@@ -126,9 +126,10 @@ struct TaskArgs {
   int* status;                 // 0 ok, 1 wait timeout
   long long wait_limit_ns;
   int wait_bias;
-  int lpc;                     // lanes per cell: 1, 2 (cells of 9 or more dofs), or 32 (one warp
-                               // per cell, sweep_wide.cuh; tiling 1 x 1 x 1, expanded source)
-  int grouped;                 // 1: the default form, lpc lanes per cell (sweep_group.cuh)
+  int lpc;                     // lanes per cell.  Explicit tilings: 1, 2 (cells of 9 or more dofs), or 32
+                               // (one warp per cell, sweep_wide.cuh; tiling 1 x 1 x 1, expanded source);
+                               // default forms: 1 (sweep_lane.cuh), 2, 4, 8, 16 or 32 (sweep_group.cuh)
+  int grouped;                 // 1: a default form
 };
 // the same with what only the default forms read
 template <typename real>

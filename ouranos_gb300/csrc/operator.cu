@@ -300,16 +300,18 @@ size_t edge_bytes(const ouranos_rt* rt, int wx, int wy) {
 //   2-D Q1 256^2 LS S16    nominal 563 / 385     1 lane  438 / 276
 //   2-D Q2 256^2 LS S16    nominal 1144 / 769    1 lane  1098 / 500   4 lanes 1220 / 577
 //   2-D Q2 100^2 LS S8     nominal 292 / 221     1 lane  305 / 176    4 lanes 278 / 174
-//   2-D Q2 40^2 LS S8      nominal 126 / 83      1 lane  139 / 82     4 lanes 108 / 72
-//   2-D Q3 135x93 LS S12   nominal 849 / 352     4 lanes 532 / 217    8 lanes 430 / 231
-//   2-D Q4 200^2 LS S12    nominal 6734 / 2982   4 lanes 2356 / 879   8 lanes 2171 / 862
-//   2-D Q5 64^2 LS S8      nominal 972 / 518     8 lanes 884 / 198    16 lanes 606 / 207
+//   2-D Q2 40^2 LS S8      nominal 126 / 83      1 lane  139 / 82     4 lanes 106 / 65
+//   2-D Q3 135x93 LS S12   nominal 849 / 352     4 lanes 532 / 217    8 lanes 421 / 225
+//   2-D Q4 200^2 LS S12    nominal 6424 / 3072   4 lanes 2356 / 879   8 lanes 1886 / 690
+//   2-D Q5 64^2 LS S8      nominal 890 / 390     8 lanes 884 / 198    16 lanes 444 / 163
 //   3-D Q1 64^3 GLC S12    nominal 4533 / 1863   1 lane  3381 / 1261  2 lanes 4953 / 1933
-//   3-D Q2 48^3 LS S8      nominal 17419 / 7391  8 lanes 6542 / 2193  16 lanes 6560 / 2740
-//   3-D Q2 16^3 LS S4      nominal 933 / 358     8 lanes 245 / 124    16 lanes 202 / 79
+//   3-D Q2 48^3 LS S8      nominal 18705 / 7483  8 lanes 5958 / 2233  16 lanes 6560 / 2740
+//   3-D Q2 16^3 LS S4      nominal 1131 / 380    8 lanes 245 / 124    16 lanes 163 / 81
 //   3-D Q3 32^3 LS S8      nominal 11977 / 5784  8 lanes 11859 / 2470 16 lanes 7469 / 2336
-//   3-D Q4 10^3 LS S4      nominal 1020 / 448    16 lanes 959 / 414   32 lanes 579 / 280
-//   3-D Q5 8^3 LS S4       nominal 2682 / 1208   32 lanes 969 / 369
+//   3-D Q4 10^3 LS S4      nominal 1038 / 420    16 lanes 959 / 414   32 lanes 493 / 112
+//   3-D Q5 8^3 LS S4       nominal 3461 / 1382   32 lanes 737 / 229
+// (the forms not taken, and 3-D Q3, before the kernels' registers were cut to three blocks
+// an SM, see group_blocks).
 // More lanes to a cell shorten a step (small problems wait on the wavefront's
 // steps), fewer spend less of it on passing b and the faces around.  A member of a
 // batch counts as a large problem: the batch's launch is full anyway, and fewer

@@ -1,6 +1,7 @@
 // Transport sweep kernel for sm_103a: the form with each cell in one lane's (or two
-// lanes') registers, run for the explicit tilings of 2-D Q1 and Q2 and 3-D Q1; the
-// default forms (sweep_lane.cuh, sweep_group.cuh) share its scheme and its bits.
+// lanes') registers, run for the explicit tilings of 2-D Q1 and Q2 and 3-D Q1, and by
+// default where a cell is solved in FP64 (larger 2-D Q2, 3-D Q1) or two moments are fused;
+// the default forms (sweep_lane.cuh, sweep_group.cuh) share its scheme and its bits.
 //
 // Replaces the reference's task loop
 //   initialize_scheduler(); while (n_tasks_to_execute) sweep(*get_next_task(), ...)

@@ -1,4 +1,5 @@
-// The sweep with H lanes to a cell: the default form of every DG order.
+// The sweep with H lanes to a cell: the default form of the orders above 2-D Q2 and
+// 3-D Q1, and of 2-D Q2 with few cells or many materials side by side.
 //
 // A task is one direction crossing a tile of G = 32 / H cells of the transverse
 // plane; lane (g, h) works on cell g = (lx, ly) and, at step s, on plane
