@@ -72,13 +72,14 @@ def workload_config(cells, directions, moments, dofs_per_cell, world):
 
 # DRAM traffic of one sweep launch on the default workload
 # (dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of the
-# default form, one lane per cell in tiles of 32, whose nominal tiling is
-# 16 x 1, in the default FP64 arithmetic), keyed by a digest of its sources at
-# the time of the capture: after any change to those sources the figure no
-# longer describes the kernel and the line reports traffic as null.
-PROFILED_TILING = (16, 1, 1)
-SWEEP_SOURCES = ("sweep_lane.cuh", "sweep_lane_df64.cu", "sweep_group.cuh", "sweep.cuh", "pack2.cuh")
-SWEEP_TRAFFIC = {"digest": "787012ed0bb8d950", "bytes": {"fp64": 696841728 + 644420864}}
+# default form, one lane per cell in tiles of 32, in the default FP64
+# arithmetic), keyed by the form and by a digest of its sources at the time of
+# the capture: after any change to those sources, or in another form, the figure
+# no longer describes the kernel and the line reports traffic as null.
+PROFILED_FORM = (32, 1, 1, 1, True)
+SWEEP_SOURCES = ("sweep_lane.cuh", "sweep_lane_df64.cu", "sweep_group.cuh", "sweep.cuh", "pack2.cuh", "df64.cuh",
+                 "launch_state.h")
+SWEEP_TRAFFIC = {"digest": "8b06e9ac3fc06918", "bytes": {"fp64": 697490944 + 644693760}}
 
 
 def sweep_source_digest():
@@ -487,10 +488,10 @@ def run_ours(args):
         native["fp32_apply"] = fp32
 
     peak, peak_kind = measured_peaks()
-    # the captured configuration only: default seed, tiling and FP64 arithmetic,
-    # and the sweep sources unchanged since the capture
+    # the captured configuration only: default seed, form and FP64 arithmetic, and
+    # the sweep sources unchanged since the capture
     digest = sweep_source_digest()
-    profiled = (rank == 0 and rt.tiling() == PROFILED_TILING and world == 1)
+    profiled = (rank == 0 and rt.form() == PROFILED_FORM and world == 1)
     fresh = digest == SWEEP_TRAFFIC["digest"]
     traffic = SWEEP_TRAFFIC["bytes"].get(args.precision) if (profiled and fresh) else None
     rb = 8 if args.precision == "fp64" else 4
